@@ -12,12 +12,21 @@
 namespace aq {
 
 #ifdef __CUDACC__
-// One box of a 2-D tensor map, global -> shared; x counts elements of the inner
+// One box of a 3-D tensor map, global -> shared; x counts elements of the inner
 // dimension and x * element size must be a multiple of 16 bytes.
-__device__ __forceinline__ void tensor_copy_2d(uint32_t dst, const CUtensorMap* map, int x, int y, uint32_t bar) {
+__device__ __forceinline__ void tensor_copy_3d(uint32_t dst, const CUtensorMap* map, int x, int y, int z, uint32_t bar) {
   asm volatile(
-      "cp.async.bulk.tensor.2d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3}], [%4];" ::"r"(dst),
-      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(bar)
+      "cp.async.bulk.tensor.3d.shared::cluster.global.tile.mbarrier::complete_tx::bytes [%0], [%1, {%2, %3, %4}], [%5];" ::"r"(dst),
+      "l"(reinterpret_cast<uint64_t>(map)), "r"(x), "r"(y), "r"(z), "r"(bar)
+      : "memory");
+}
+// One box shared -> global; boxes are cut at the borders of the map.  The copy joins this thread's
+// bulk group, which is closed here.
+__device__ __forceinline__ void tensor_store_2d(const CUtensorMap* map, int x, int y, uint32_t src) {
+  asm volatile(
+      "cp.async.bulk.tensor.2d.global.shared::cta.tile.bulk_group [%0, {%1, %2}], [%3];\n\t"
+      "cp.async.bulk.commit_group;" ::"l"(reinterpret_cast<uint64_t>(map)),
+      "r"(x), "r"(y), "r"(src)
       : "memory");
 }
 __device__ __forceinline__ void tc_fence_before() {
@@ -35,8 +44,8 @@ __device__ __forceinline__ void tc_mma_i8(uint32_t d_tmem, uint64_t a_desc, uint
   asm volatile(
       "{\n\t.reg .pred p;\n\t"
       "setp.ne.b32 p, %4, 0;\n\t"
-      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, {%5, %5, %5, %5}, p;\n\t}" ::"r"(d_tmem),
-      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate), "r"(0u)
+      "tcgen05.mma.cta_group::1.kind::i8 [%0], %1, %2, %3, p;\n\t}" ::"r"(d_tmem),
+      "l"(a_desc), "l"(b_desc), "r"(idesc), "r"(accumulate)
       : "memory");
 }
 __device__ __forceinline__ void tc_ld16(uint32_t taddr, int (&v)[16]) {
@@ -55,6 +64,28 @@ __device__ __forceinline__ void tc_wait_ld(int (&v)[16]) {
   asm volatile("tcgen05.wait::ld.sync.aligned;"
                : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
                  "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15])
+               :
+               : "memory");
+}
+// 32 columns at once: 32 registers per lane.
+__device__ __forceinline__ void tc_ld32(uint32_t taddr, int (&v)[32]) {
+  asm volatile(
+      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
+      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
+      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
+      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
+        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
+        "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
+        "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
+      : "r"(taddr)
+      : "memory");
+}
+__device__ __forceinline__ void tc_wait_ld32(int (&v)[32]) {
+  asm volatile("tcgen05.wait::ld.sync.aligned;"
+               : "+r"(v[0]), "+r"(v[1]), "+r"(v[2]), "+r"(v[3]), "+r"(v[4]), "+r"(v[5]), "+r"(v[6]), "+r"(v[7]),
+                 "+r"(v[8]), "+r"(v[9]), "+r"(v[10]), "+r"(v[11]), "+r"(v[12]), "+r"(v[13]), "+r"(v[14]), "+r"(v[15]),
+                 "+r"(v[16]), "+r"(v[17]), "+r"(v[18]), "+r"(v[19]), "+r"(v[20]), "+r"(v[21]), "+r"(v[22]), "+r"(v[23]),
+                 "+r"(v[24]), "+r"(v[25]), "+r"(v[26]), "+r"(v[27]), "+r"(v[28]), "+r"(v[29]), "+r"(v[30]), "+r"(v[31])
                :
                : "memory");
 }
@@ -141,18 +172,42 @@ inline EncodeTiledFn encode_tiled_fn() {
   return g_encode_tiled;
 }
 
-// Row-major int8 [m][k] seen as boxes of box_rows rows x 64 bytes that land with the 64-byte
-// swizzle; rows past m are filled with zeros.
-inline int encode_activation_map(CUtensorMap* map, const int8_t* xq, int64_t m, int64_t k, int box_rows) {
+// Row-major int8 [m][64 n_k] seen as [n_k][m][64], in boxes of box_steps x box_rows x 64 bytes that
+// land with the 64-byte swizzle; rows past m and steps past n_k are filled with zeros.
+inline int encode_activation_map(CUtensorMap* map, const int8_t* xq, int64_t m, int n_k, int box_rows, int box_steps) {
   EncodeTiledFn encode = encode_tiled_fn();
   if (encode == nullptr) return fail(AQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
-  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(k), static_cast<cuuint64_t>(m)};
-  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(k)};
-  const cuuint32_t box[2] = {static_cast<cuuint32_t>(kTile), static_cast<cuuint32_t>(box_rows)};
-  const cuuint32_t elem_strides[2] = {1, 1};
-  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 2, const_cast<int8_t*>(xq), dims, strides, box,
+  const cuuint64_t dims[3] = {static_cast<cuuint64_t>(kTile), static_cast<cuuint64_t>(m), static_cast<cuuint64_t>(n_k)};
+  const cuuint64_t strides[2] = {static_cast<cuuint64_t>(n_k) * kTile, static_cast<cuuint64_t>(kTile)};
+  const cuuint32_t box[3] = {static_cast<cuuint32_t>(kTile), static_cast<cuuint32_t>(box_rows), static_cast<cuuint32_t>(box_steps)};
+  const cuuint32_t elem_strides[3] = {1, 1, 1};
+  const CUresult r = encode(map, CU_TENSOR_MAP_DATA_TYPE_UINT8, 3, const_cast<int8_t*>(xq), dims, strides, box,
                             elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_64B,
                             CU_TENSOR_MAP_L2_PROMOTION_L2_128B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) return fail(AQ_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", static_cast<int>(r));
+  return AQ_OK;
+}
+
+// Row-major results [m][n] in boxes of box_rows rows x up to box_cols columns, at most 128 bytes of a
+// row: no swizzle for 16 columns, else the 128-byte swizzle for 128-byte boxes and the 64-byte one for
+// 64-byte boxes.
+inline int encode_result_map(CUtensorMap* map, void* out, int out_dtype, int64_t m, int64_t n, int box_cols, int box_rows) {
+  EncodeTiledFn encode = encode_tiled_fn();
+  if (encode == nullptr) return fail(AQ_ERR_CUDA, "cuTensorMapEncodeTiled is not available from this driver");
+  const int size = out_dtype == AQ_F32 ? 4 : 2;
+  if (box_cols * size > 128) box_cols = 128 / size;
+  const CUtensorMapDataType type = out_dtype == AQ_F32    ? CU_TENSOR_MAP_DATA_TYPE_FLOAT32
+                                   : out_dtype == AQ_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16
+                                                          : CU_TENSOR_MAP_DATA_TYPE_FLOAT16;
+  const cuuint64_t dims[2] = {static_cast<cuuint64_t>(n), static_cast<cuuint64_t>(m)};
+  const cuuint64_t strides[1] = {static_cast<cuuint64_t>(n) * size};
+  const cuuint32_t box[2] = {static_cast<cuuint32_t>(box_cols), static_cast<cuuint32_t>(box_rows)};
+  const cuuint32_t elem_strides[2] = {1, 1};
+  const CUresult r = encode(map, type, 2, out, dims, strides, box, elem_strides, CU_TENSOR_MAP_INTERLEAVE_NONE,
+                            box_cols == 16           ? CU_TENSOR_MAP_SWIZZLE_NONE
+                            : box_cols * size == 128 ? CU_TENSOR_MAP_SWIZZLE_128B
+                                                     : CU_TENSOR_MAP_SWIZZLE_64B,
+                            CU_TENSOR_MAP_L2_PROMOTION_NONE, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
   if (r != CUDA_SUCCESS) return fail(AQ_ERR_CUDA, "cuTensorMapEncodeTiled failed with code %d", static_cast<int>(r));
   return AQ_OK;
 }

@@ -480,18 +480,30 @@ def alignquant_quant_linear(
 
 
 _WORKSPACES: dict[tuple, torch.Tensor] = {}
+_WORKSPACE_POOLS: dict[int, "torch.cuda.MemPool"] = {}
+_WORKSPACE_MOST = (64 << 20) + (64 << 10)  # most that a GEMM asks for (aq_linear_workspace_bytes): taken at once
 
 
 def _workspace(device: torch.device, size: int) -> torch.Tensor:
-    """Zeroed scratch for split-K partials, one per (device, stream).
+    """Zeroed scratch for split-K partials and the GEMM's expanded weights, one per (device, stream).
 
-    The kernels leave the workspace zeroed, and calls on one stream run in order, so a
-    single buffer per stream is reused by every call; it only grows.
+    The kernels leave the counters at its start zeroed, and calls on one stream run in order, so a
+    single buffer per stream is reused by every call; it only grows, to at most 64 MiB and a little.
+    It comes from a memory pool of its own: a buffer of this size that lives on inside a segment of
+    the general pool would keep the rest of that segment from being returned.
     """
     key = (device.index, _stream(device))
     buffer = _WORKSPACES.get(key)
     if buffer is None or buffer.numel() < size:
-        buffer = torch.zeros((max(size, 1 << 21),), dtype=torch.uint8, device=device)
+        size = max(size, 1 << 21 if size <= 1 << 21 else _WORKSPACE_MOST)
+        if torch.cuda.is_current_stream_capturing():  # a capture brings its own pool
+            buffer = torch.zeros((size,), dtype=torch.uint8, device=device)
+        else:
+            pool = _WORKSPACE_POOLS.get(device.index)
+            if pool is None:
+                pool = _WORKSPACE_POOLS.setdefault(device.index, torch.cuda.MemPool())
+            with torch.cuda.use_mem_pool(pool, device):
+                buffer = torch.zeros((size,), dtype=torch.uint8, device=device)
         _WORKSPACES[key] = buffer
     return buffer
 

@@ -68,10 +68,10 @@ AQ_API int aq_version(void);
  *                           (alignquant/kernels/cuda/linear.cu:956-963), about 20 % slower.  The
  *                           per-tile int32 sums are exact either way.
  *   AQ_OPT_GEMM_TILE        CTA tile of the GEMM, for tests and measurements: AQ_GEMM_TILE_AUTO
- *                           (default), AQ_GEMM_TILE_PAIRED (128 columns, two 256-thread CTAs per
- *                           SM), AQ_GEMM_TILE_NARROW (128 columns, one 512-thread CTA per SM),
- *                           AQ_GEMM_TILE_WIDE (256 columns, one CTA per SM).  Results are
- *                           bit-identical across the three.
+ *                           (default), AQ_GEMM_TILE_PAIRED (128 columns, two K steps per hand-over),
+ *                           AQ_GEMM_TILE_NARROW (192 columns), AQ_GEMM_TILE_WIDE (256 columns).
+ *                           Results are bit-identical across the three.  (Layers with an output
+ *                           transform and a single K range always run 256 columns wide.)
  *   AQ_OPT_GEMM_SPLIT       number of K ranges of the GEMM (1..8), 0 = automatic (default); changes
  *                           the FP32 summation order as aq_linear_plan reports.
  *   AQ_OPT_DECODE_KERNEL    AQ_DECODE_KERNEL_AUTO (default); AQ_DECODE_KERNEL_CLUSTER: never use
@@ -174,7 +174,8 @@ AQ_API int aq_repack(const uint8_t* state_bits, const uint8_t* w4_payload, const
 /*
  * Bytes of workspace aq_linear needs for this problem (0 when none is needed).  The
  * workspace holds per-row arrival counters (its first 64 KiB) followed by split-K
- * partial tiles.  Its owner must zero it once before the first call; every call
+ * partial tiles or, for the GEMM, weights expanded to int8 (at most 64 MiB: larger layers are
+ * run in several passes over their columns).  Its owner must zero it once before the first call; every call
  * returns the counters to zero, so one buffer can be reused by later calls on the same
  * stream, for any layer.  Calls that may run concurrently (other
  * streams) need separate workspaces.  After an AQ_ERR_DEVICE report zero it again.

@@ -167,3 +167,23 @@ def test_gemm_split_k_clusters(options, m, split):
     xq_np = xq.cpu().numpy()
     assert np.array_equal(dump.cpu().numpy(), oc.tile_accumulators_c(xq_np, tiles))
     assert np.array_equal(out.cpu().numpy(), oc.linear_fp32_c(xq_np, a_mk, tiles, scales, int(split), fused=True))
+
+
+@pytest.mark.parametrize("tile", ["paired", "narrow", "wide", "auto"])
+@pytest.mark.parametrize("m,n,k", [(1190, 2368, 192), (33, 2624, 32768), (1999, 1088, 64)])
+def test_gemm_many_tiles_per_cta_and_column_passes(options, tile, m, n, k):
+    """More output tiles than SMs (a CTA walks several, with an odd number of K steps and ragged last
+    row and column blocks), a layer above the 64 MiB of expanded weights (several passes over its
+    columns) and a single K step; every result type through the tensor-map stores.  FP32 sums are
+    compared bit for bit, the 16-bit results with their rounding of them."""
+    ext = options
+    ext.set_gemm_tile(tile)
+    ext.set_gemm_split(1)
+    weights, tiles, scales, xq, a_s, a_mk = _case(ext, m, n, k, "token", seed=m + n)
+    xq_np = xq.cpu().numpy()
+    want = torch.from_numpy(oc.linear_fp32_c(xq_np, a_mk, tiles, scales, 1, fused=True))
+    for dtype in (torch.float32, torch.bfloat16, torch.float16):
+        out = ext.alignquant_linear_prepared(xq, a_s, weights, None, schedule="forced_prefill_m64", scale_mode="token",
+                                             output_dtype=dtype)
+        ext.device_status()
+        assert torch.equal(out.cpu(), want.to(dtype))
