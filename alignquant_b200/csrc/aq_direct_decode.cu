@@ -331,10 +331,9 @@ __global__ void __launch_bounds__(32 * WARPS, NG == 1 ? 3 : 2) direct_decode_ker
       for (int v = threadIdx.x; v < vectors_per_row; v += kThreads) {
         float f[8];
         unpack8(__ldg(raw_global + static_cast<int64_t>(r) * vectors_per_row + v), raw_bf16, f);
-        int q8[8];
-#pragma unroll
-        for (int i = 0; i < 8; ++i) q8[i] = quantize_token_value(f[i], scale, inv_scale);
-        const uint32_t lo = pack4(q8[0], q8[1], q8[2], q8[3]), hi = pack4(q8[4], q8[5], q8[6], q8[7]);
+        const auto exact = [=](float value) { return quantize_token_value(value, scale, inv_scale); };
+        const uint32_t lo = quantize4(f[0], f[1], f[2], f[3], inv_scale, exact);
+        const uint32_t hi = quantize4(f[4], f[5], f[6], f[7], inv_scale, exact);
         asm volatile("st.shared.v2.u32 [%0], {%1, %2};" ::"r"(x_stage + static_cast<uint32_t>(r) * x_stride + static_cast<uint32_t>(v) * 8u),
                      "r"(lo), "r"(hi)
                      : "memory");

@@ -28,6 +28,28 @@ __device__ __forceinline__ uint32_t pack4(int a, int b, int c, int d) {
          ((static_cast<uint32_t>(c) & 0xffu) << 16) | ((static_cast<uint32_t>(d) & 0xffu) << 24);
 }
 
+// Four values -> four int8 codes.  v * inv is rounded to a whole number by adding 1.5 * 2^23 (one
+// fused multiply-add; the code is the low byte of the sum), the distance to it by a second one.  The
+// callers' inv differs from 1 / scale by less than 2^-22 of it and |v / scale| < 129, so the distance
+// is off by less than 4e-5: below 0.5 - 1e-4 the code is that of the exact quotient and lies in
+// the code's range.  Otherwise (and for NaN) all four go to `exact`.  Full-rate instructions only:
+// conversions to and from integers run at a quarter of the rate and, with the compares, clamps and
+// masks of quantize_token_value, bounded the quantizers (8192 x 8192 bf16: 59 us).
+template <typename Exact>
+__device__ __forceinline__ uint32_t quantize4(float v0, float v1, float v2, float v3, float inv, Exact exact) {
+  constexpr float kMagic = 12582912.0f, kClear = 0.5f - 1.0e-4f;
+  const float m0 = __fmaf_rn(v0, inv, kMagic), m1 = __fmaf_rn(v1, inv, kMagic);
+  const float m2 = __fmaf_rn(v2, inv, kMagic), m3 = __fmaf_rn(v3, inv, kMagic);
+  const float d0 = __fmaf_rn(v0, inv, __fsub_rn(kMagic, m0)), d1 = __fmaf_rn(v1, inv, __fsub_rn(kMagic, m1));
+  const float d2 = __fmaf_rn(v2, inv, __fsub_rn(kMagic, m2)), d3 = __fmaf_rn(v3, inv, __fsub_rn(kMagic, m3));
+  if (fabsf(d0) <= kClear && fabsf(d1) <= kClear && fabsf(d2) <= kClear && fabsf(d3) <= kClear) {
+    const uint32_t lo = __byte_perm(__float_as_uint(m0), __float_as_uint(m1), 0x0040);
+    const uint32_t hi = __byte_perm(__float_as_uint(m2), __float_as_uint(m3), 0x0040);
+    return __byte_perm(lo, hi, 0x5410);
+  }
+  return pack4(exact(v0), exact(v1), exact(v2), exact(v3));
+}
+
 // Eight fp16 or bf16 values (one 16-byte vector) as floats.
 __device__ __forceinline__ void unpack8(const uint4& raw, bool bf16, float (&v)[8]) {
   const uint32_t w[4] = {raw.x, raw.y, raw.z, raw.w};

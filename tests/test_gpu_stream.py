@@ -136,6 +136,32 @@ def _run_linear(ext, xq, a_s, weights, u_meta, m, n_j, n_k, **kw):
     return out, dump
 
 
+@pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
+@pytest.mark.parametrize("m,k", [(1024, 512), (1025, 64), (1031, 512), (1025, 576), (1025, 1024), (1027, 1088), (1026, 4096),
+                                 (1025, 4160), (3, 2048), (3, 2112), (5, 8192), (3, 8256), (2, 16384), (2, 16448), (2, 32768), (2, 32832)])
+def test_row_quantizers_at_the_borders_of_their_layouts(ext, m, k, dtype):
+    """Every number of warps per row and of vectors per lane, with the last lanes full and nearly empty, and
+    rows of zeros, infinities and NaN, whose codes and scales follow fmaxf, IEEE division and the int conversion."""
+    gen = torch.Generator(device="cuda").manual_seed(m + k)
+    x = torch.randn(m, k, generator=gen, device="cuda").to(dtype)
+    x[0] = 0
+    x[1, k // 2], x[1, 3] = float("inf"), float("nan")
+    q, s = ext.alignquant_activation_quantize_cuda(x, None, scale_mode="token")
+    f = x.float()
+    most = torch.nan_to_num(f, nan=0.0, posinf=float("inf"), neginf=-float("inf")).abs().amax(1)
+    scale = (most / torch.full_like(most, 127.0)).clamp_min(1e-12)  # by a tensor: torch multiplies by a scalar's reciprocal
+    codes = torch.nan_to_num(torch.round(f / scale[:, None]), nan=0.0).clamp(-127, 127).to(torch.int8)
+    assert torch.equal(s, scale) and torch.equal(q, codes)
+    weight = (1.0 + 0.1 * torch.randn(k, generator=gen, device="cuda")).to(dtype)
+    normed = torch.empty_like(x)
+    q, s = ext.alignquant_rmsnorm_quantize_cuda(x, weight, 1e-6, normed=normed)
+    r = (1.0 / torch.sqrt(x.double().pow(2).mean(1) + 1e-6)).float()
+    y = (weight.float() * (f * r[:, None]).to(dtype).float()).to(dtype)
+    assert torch.equal(normed[2:], y[2:]) and bool((normed[0] == 0).all()) and bool(normed[1].isnan().all())
+    want = ext.alignquant_activation_quantize_cuda(normed, None, scale_mode="token")
+    assert torch.equal(q, want[0]) and torch.equal(s, want[1])
+
+
 @pytest.mark.parametrize("scale_mode", ["tile", "token"])
 @pytest.mark.parametrize("m", [1, 4, 16, 17, 32, 33, 64, 128])
 @pytest.mark.parametrize("n,k", [(64, 64), (128, 192), (192, 512)])
