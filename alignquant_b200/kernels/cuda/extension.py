@@ -14,6 +14,7 @@ counts that are not multiples of 16, and ``prepare_weights`` /
 
 from __future__ import annotations
 
+import contextlib
 import weakref
 from dataclasses import dataclass
 
@@ -36,13 +37,21 @@ def load_extension() -> None:
 
 
 def _stream(device: torch.device) -> int:
-    return int(torch.cuda.current_stream(device).cuda_stream)
+    # the stream's handle itself; torch.cuda.current_stream builds an object around it (1.3 us)
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if device.index is None else device.index)
+
+
+_SAME_DEVICE = contextlib.nullcontext()
+
+
+def _on(device: torch.device):
+    """``torch.cuda.device(device)`` where that changes anything."""
+    return _SAME_DEVICE if torch.cuda.current_device() == device.index else torch.cuda.device(device)
 
 
 def _ptr(tensor: torch.Tensor | None) -> int | None:
-    if tensor is None or tensor.numel() == 0:
-        return None
-    return int(tensor.data_ptr())
+    # a tensor without elements has a null pointer, or none of its own
+    return (tensor.data_ptr() or None) if tensor is not None and tensor.numel() else None
 
 
 def _require_cuda(tensor: torch.Tensor, name: str) -> None:
@@ -103,7 +112,7 @@ def alignquant_activation_quantize_cuda(
             meta = None
     n_m = (m + 15) // 16
     scale_shape = (m,) if mode == _lib.AQ_SCALE_TOKEN else ((n_k,) if n_m == 1 else (n_m, n_k))
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         if out is not None:
             q, scales = out
             if (q.dtype != torch.int8 or tuple(q.shape) != (m, k) or not q.is_contiguous()
@@ -149,7 +158,7 @@ def alignquant_rmsnorm_quantize_cuda(
     m, k = int(x.size(0)), int(x.size(1))
     if k % 64 or tuple(w.shape) != (k,) or w.device != x.device:
         raise RuntimeError("K must be a multiple of 64 and weight must be [K] on x's device")
-    with torch.cuda.device(x.device):
+    with _on(x.device):
         if out is not None:
             q, scales = out
             if (q.dtype != torch.int8 or tuple(q.shape) != (m, k) or not q.is_contiguous() or scales.dtype != torch.float32
@@ -245,7 +254,7 @@ def prepare_weights(
     size = int(lib.aq_prepared_bytes(n_j, n_k, t4, t8))
     if size < 0:
         _lib.check(size)
-    with torch.cuda.device(device):
+    with _on(device):
         image = torch.empty((size,), dtype=torch.uint8, device=device)
         keep = [t.contiguous() for t, _ in tensors.values()]
         _lib.check(
@@ -329,15 +338,15 @@ def alignquant_linear_prepared(
         if acc_dump.dtype != torch.int32 or tuple(acc_dump.shape) != (m, n_j, n_k, 64) or not acc_dump.is_contiguous():
             raise RuntimeError("acc_dump must be a contiguous int32 [M,N/64,K/64,64] tensor")
     lib = _lib.load()
-    with torch.cuda.device(device):
+    with _on(device):
         if out is None:
             out = torch.empty((m, n_j * 64), dtype=output_dtype, device=device)
         elif out.dtype != output_dtype or tuple(out.shape) != (m, n_j * 64) or not out.is_contiguous():
             raise RuntimeError("out must be a contiguous [M,N] tensor of output_dtype")
-        ws_bytes = int(lib.aq_linear_workspace_bytes(m, n_j, n_k, schedule_code, int(decode_splits)))
+        ws_bytes = lib.aq_linear_workspace_bytes(m, n_j, n_k, schedule_code, int(decode_splits))
         if ws_bytes < 0:
             _lib.check(ws_bytes)
-        workspace = _workspace(device, ws_bytes) if ws_bytes else None
+        workspace = _workspace(device, ws_bytes, _takes_gemm(m, schedule_code)) if ws_bytes else None
         if prefetch is not None and prefetch.device != device:
             raise RuntimeError("prefetch must name weights on the device of this call")
         _lib.check(
@@ -383,7 +392,7 @@ def alignquant_linear_allreduce(
     device = x.device
     meta = None if u_metadata is None else u_metadata.contiguous()
     lib = _lib.load()
-    with torch.cuda.device(device):
+    with _on(device):
         if out is None:
             out = torch.empty((m, n_j * 64), dtype=output_dtype, device=device)
         _lib.check(
@@ -445,31 +454,33 @@ def alignquant_quant_linear(
             raise RuntimeError("u_metadata must be int32 [N/64,4,64] on x's device")
         meta = u_metadata.contiguous()
     lib = _lib.load()
-    with torch.cuda.device(device):
+    with _on(device):
         if quantized is not None:
             q, scales = quantized
             if (q.dtype != torch.int8 or tuple(q.shape) != (m, k) or not q.is_contiguous() or scales.dtype != torch.float32
                     or tuple(scales.shape) != (m,) or not scales.is_contiguous() or q.device != device or scales.device != device):
                 raise RuntimeError("quantized must be (contiguous int8 [M,K], contiguous float32 [M]) on x's device")
-        else:
-            q = torch.empty((m, k), dtype=torch.int8, device=device)
-            scales = torch.empty((m,), dtype=torch.float32, device=device)
+            q_ptr, scales_ptr = _ptr(q), _ptr(scales)
+        else:  # nobody else sees them: one allocation, the scales behind the codes (m K is a multiple of 64)
+            q = torch.empty((m * (k + 4),), dtype=torch.int8, device=device)
+            q_ptr = q.data_ptr()
+            scales_ptr = q_ptr + m * k
         if out is None:
             out = torch.empty((m, n_j * 64), dtype=output_dtype, device=device)
         elif out.dtype != output_dtype or tuple(out.shape) != (m, n_j * 64) or not out.is_contiguous():
             raise RuntimeError("out must be a contiguous [M,N] tensor of output_dtype")
         ws_bytes, workspace = 0, None
         if reducer is None:
-            ws_bytes = int(lib.aq_linear_workspace_bytes(m, n_j, n_k, _lib.SCHEDULE_CODES["auto"], 0))
+            ws_bytes = lib.aq_linear_workspace_bytes(m, n_j, n_k, 0, 0)
             if ws_bytes < 0:
                 _lib.check(ws_bytes)
-            workspace = _workspace(device, ws_bytes) if ws_bytes else None
+            workspace = _workspace(device, ws_bytes, _takes_gemm(m, 0)) if ws_bytes else None
         if prefetch is not None and prefetch.device != device:
             raise RuntimeError("prefetch must name weights on the device of this call")
         _lib.check(
             lib.aq_quant_linear(
                 _ptr(x), _DTYPE_CODES[x.dtype], m, _ptr(weights.image), n_j, n_k, _ptr(meta), _DTYPE_CODES[output_dtype],
-                _ptr(out), _ptr(q), _ptr(scales), _ptr(workspace), ws_bytes,
+                _ptr(out), q_ptr, scales_ptr, _ptr(workspace), ws_bytes,
                 0 if reducer is None else reducer.rank, 1 if reducer is None else reducer.world,
                 None if reducer is None else reducer.peer_array_pointer(), 0 if reducer is None else reducer.max_count,
                 None if prefetch is None else _ptr(prefetch.image),
@@ -480,30 +491,27 @@ def alignquant_quant_linear(
 
 
 _WORKSPACES: dict[tuple, torch.Tensor] = {}
-_WORKSPACE_POOLS: dict[int, "torch.cuda.MemPool"] = {}
-_WORKSPACE_MOST = (64 << 20) + (64 << 10)  # most that a GEMM asks for (aq_linear_workspace_bytes): taken at once
 
 
-def _workspace(device: torch.device, size: int) -> torch.Tensor:
-    """Zeroed scratch for split-K partials and the GEMM's expanded weights, one per (device, stream).
+def _takes_gemm(m: int, schedule_code: int) -> bool:
+    """Which of the two kernels with a workspace a call takes; the stream-K kernel has at most 16 rows."""
+    return m > 16 or schedule_code == _lib.SCHEDULE_CODES["forced_prefill_m64"]
 
-    The kernels leave the counters at its start zeroed, and calls on one stream run in order, so a
-    single buffer per stream is reused by every call; it only grows, to at most 64 MiB and a little.
-    It comes from a memory pool of its own: a buffer of this size that lives on inside a segment of
-    the general pool would keep the rest of that segment from being returned.
+
+def _workspace(device: torch.device, size: int, gemm: bool) -> torch.Tensor:
+    """Scratch of one call.
+
+    The GEMM's (``gemm``: expanded weights, up to 64 MiB) needs no content: it is the caching
+    allocator's, taken and given back by every call like any temporary, so that streams, threads and captured graphs
+    never meet in it.  The stream-K kernel's holds arrival counters that a call finds and leaves
+    zeroed: one zeroed buffer per (device, stream), where calls run in order, which only grows.
     """
+    if gemm:
+        return torch.empty((size,), dtype=torch.uint8, device=device)
     key = (device.index, _stream(device))
     buffer = _WORKSPACES.get(key)
     if buffer is None or buffer.numel() < size:
-        size = max(size, 1 << 21 if size <= 1 << 21 else _WORKSPACE_MOST)
-        if torch.cuda.is_current_stream_capturing():  # a capture brings its own pool
-            buffer = torch.zeros((size,), dtype=torch.uint8, device=device)
-        else:
-            pool = _WORKSPACE_POOLS.get(device.index)
-            if pool is None:
-                pool = _WORKSPACE_POOLS.setdefault(device.index, torch.cuda.MemPool())
-            with torch.cuda.use_mem_pool(pool, device):
-                buffer = torch.zeros((size,), dtype=torch.uint8, device=device)
+        buffer = torch.zeros((max(size, 1 << 21),), dtype=torch.uint8, device=device)
         _WORKSPACES[key] = buffer
     return buffer
 
@@ -572,7 +580,7 @@ def alignquant_linear_cuda(
 def device_status(device: torch.device | str | None = None) -> None:
     """Synchronise the current stream and raise if a kernel gave up a device-side wait."""
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
-    with torch.cuda.device(dev):
+    with _on(dev):
         status = _lib.load().aq_device_status(_stream(dev))
         if status != _lib.AQ_OK:
             _WORKSPACES.clear()  # arrival counters may be left non-zero by an aborted kernel
@@ -615,7 +623,7 @@ def alignquant_linear_decode_static(
         raise RuntimeError("activation_scales has the wrong dtype or size for this scale_mode")
     device = x.device
     meta = None if u_metadata is None else u_metadata.contiguous()
-    with torch.cuda.device(device):
+    with _on(device):
         if out is None:
             out = torch.empty((m, n_j * 64), dtype=output_dtype, device=device)
         _lib.check(
@@ -672,7 +680,7 @@ def measure_int8_peak(pairs: int = 4096, device: torch.device | str | None = Non
 
     dev = torch.device("cuda", torch.cuda.current_device()) if device is None else torch.device(device)
     tops = ctypes.c_double()
-    with torch.cuda.device(dev):
+    with _on(dev):
         _lib.check(_lib.load().aq_measure_int8_peak(int(pairs), ctypes.addressof(tops), _stream(dev)))
     return float(tops.value)
 

@@ -227,11 +227,8 @@ class _ProjectionGroupRuntime:
 
     @staticmethod
     def _activation_key(activation: torch.Tensor) -> tuple[Any, ...]:
-        return (
-            activation.device.type, activation.device.index, activation.data_ptr(),
-            int(activation.storage_offset()), tuple(int(v) for v in activation.shape),
-            tuple(int(v) for v in activation.stride()), str(activation.dtype),
-        )
+        return (activation.device, activation.data_ptr(), activation.storage_offset(), activation.shape,
+                activation.stride(), activation.dtype)
 
     def project_member(self, activation: torch.Tensor, *, member: str) -> tuple[torch.Tensor, tuple[int, ...]]:
         """Slice of the group's output that belongs to ``member``, computing the group once."""
@@ -258,7 +255,7 @@ class _ProjectionGroupRuntime:
                 raise ValueError(f"Projection group {self.group_id} is on {self.device}, got {activation.device}.")
             if activation.dim() < 1:
                 raise ValueError(f"Native W4/W8A8 linear expects [...,K], got {tuple(activation.shape)}.")
-            original_shape = tuple(int(v) for v in activation.shape)
+            original_shape = tuple(activation.shape)
             width = original_shape[-1]
             if width != self.n_k * 64:
                 raise ValueError(f"Activation K mismatch for {self.group_id}: {width} vs {self.n_k * 64}.")
