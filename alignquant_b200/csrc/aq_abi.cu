@@ -536,7 +536,9 @@ int aq_device_status(void* stream) {
   const int rc = check_cuda(cudaStreamSynchronize(static_cast<cudaStream_t>(stream)), "cudaStreamSynchronize");
   if (rc != AQ_OK) return rc;
   const int stream_status = take_stream_status();
-  const int gemm_status = take_gemm_status();
+  int gemm_status = take_gemm_status();
+  const int gemm_rows_status = take_gemm_rows_status();
+  if (gemm_status == 0) gemm_status = gemm_rows_status;
   const int decode_status = take_decode_status();
   const int direct_status = take_direct_decode_status();
   int cluster_decode_status = take_cluster_decode_status();

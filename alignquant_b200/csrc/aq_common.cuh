@@ -130,6 +130,13 @@ int launch_tmem_gemm(const LinearArgs& a, cudaStream_t stream);
 int64_t tmem_gemm_workspace_bytes(int64_t m, int n_j, int n_k);
 int tmem_gemm_split(int64_t m, int n_j, int n_k);  // K ranges (cluster size) the GEMM will use
 
+// GEMM for up to 128 rows that reads the packed weights once (what launch_tmem_gemm runs where it applies).
+bool gemm_rows_supported(int64_t m, int n_j, int n_k);
+int gemm_rows_split(int64_t m, int n_j, int n_k, double* cost);  // K ranges, and the modelled SM cycles
+double tmem_gemm_cost(int64_t m, int n_j, int n_k);  // the same for the GEMM with expanded weights
+int launch_gemm_rows(const LinearArgs& a, cudaStream_t stream);
+int take_gemm_rows_status();
+
 // Rate of back-to-back tcgen05.mma kind::i8 on all SMs (measurement aid; synchronises).
 int measure_int8_peak(int pairs, double* tops, cudaStream_t stream);
 

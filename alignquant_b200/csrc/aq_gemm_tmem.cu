@@ -718,9 +718,12 @@ constexpr int64_t kScratchOffset = 64 * 1024;
 // which finds its operand in the L2.
 constexpr int64_t kScratchBytes = 64LL << 20;
 
+// Tile rows per pass, the passes of about one size: the tile width and the K ranges are chosen for a pass.
 int rows_per_pass(int n_j, int n_k) {
   const int64_t most = kScratchBytes / (static_cast<int64_t>(n_k) * kW8TileBytes) / 12 * 12;  // whole CTA tiles of every width
-  return most < n_j ? static_cast<int>(most) : n_j;
+  if (most >= n_j) return n_j;
+  const int64_t passes = (n_j + most - 1) / most;
+  return static_cast<int>(((n_j + passes - 1) / passes + 11) / 12 * 12);
 }
 
 int launch_expand(const TileRecord* records, const uint8_t* payload, int n_k, int j_base, int rows, int tn, uint8_t* operand,
@@ -839,6 +842,7 @@ int device_sm_count(int* count) {
 struct Choice {
   int tn;
   int split;
+  double cost;  // modelled SM cycles of a pass
 };
 
 // The cheapest of the three tile widths and up to eight K ranges by a model in SM cycles: a CTA's K
@@ -847,6 +851,7 @@ struct Choice {
 // 4000 per tile row.  The wide tile wins where there are many output tiles (16384 x 19456 x 2560: 1287 us
 // against 1537 and 1575); the others where it would leave most of a last wave idle (2048 x 5120 x 3072:
 // 69 us against 77); K ranges only pay for a few row blocks (128 x 5120 x 3072: 16 us against 21).
+// `n_j`: tile rows of a pass (with the whole layer's, 34816 x 5120 at 48 rows ran three passes of 48 CTAs).
 // AQ_OPT_GEMM_TILE and AQ_OPT_GEMM_SPLIT force a choice.
 Choice choose(int64_t m, int n_j, int n_k, int sm_count, int device) {
   const int forced_tile = gemm_tile_option();
@@ -854,7 +859,7 @@ Choice choose(int64_t m, int n_j, int n_k, int sm_count, int device) {
   const int64_t m_blocks = (m + kBM - 1) / kBM;
   static const double kStep[5] = {0, 0, 527, 730, 850};
   static const double kHandOver[5] = {0, 0, 1400, 3000, 1800};
-  Choice best = {4, 1};
+  Choice best = {4, 1, 0.0};
   double best_cost = 0.0;
   for (int tn = 4; tn >= 2; --tn) {
     if (forced_tile == AQ_GEMM_TILE_WIDE && tn != 4) continue;
@@ -874,7 +879,7 @@ Choice choose(int64_t m, int n_j, int n_k, int sm_count, int device) {
       const double cost = static_cast<double>(waves) * ((n_k + split - 1) / split * kStep[tn] + kHandOver[tn]) + (split > 1 ? 4000.0 * tn : 0.0);
       if (best_cost == 0.0 || cost < best_cost) {
         best_cost = cost;
-        best = {tn, split};
+        best = {tn, split, cost};
       }
     }
   }
@@ -884,17 +889,30 @@ Choice choose(int64_t m, int n_j, int n_k, int sm_count, int device) {
 
 }  // namespace
 
-int64_t tmem_gemm_workspace_bytes(int64_t, int n_j, int n_k) {
+int64_t tmem_gemm_workspace_bytes(int64_t m, int n_j, int n_k) {
+  if (gemm_rows_supported(m, n_j, n_k)) return 0;
   const int64_t rows = (rows_per_pass(n_j, n_k) + 11) / 12 * 12;
   return kScratchOffset + rows * n_k * kW8TileBytes;
 }
 
-int tmem_gemm_split(int64_t m, int n_j, int n_k) {
+// Expansion (2.1 cycles per tile, measured: 14 us for 12288 tiles) and GEMM, pass by pass.
+double tmem_gemm_cost(int64_t m, int n_j, int n_k) {
   int sm_count = 148;
   if (device_sm_count(&sm_count) != AQ_OK) sm_count = 148;
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess) device = 0;
-  return choose(m, n_j, n_k, sm_count, device).split;
+  const int rows = rows_per_pass(n_j, n_k);
+  const int passes = (n_j + rows - 1) / rows;
+  return passes * choose(m, rows, n_k, sm_count, device).cost + 2.1 * static_cast<double>(n_j) * n_k + 2000.0;
+}
+
+int tmem_gemm_split(int64_t m, int n_j, int n_k) {
+  if (gemm_rows_supported(m, n_j, n_k)) return gemm_rows_split(m, n_j, n_k, nullptr);
+  int sm_count = 148;
+  if (device_sm_count(&sm_count) != AQ_OK) sm_count = 148;
+  int device = 0;
+  if (cudaGetDevice(&device) != cudaSuccess) device = 0;
+  return choose(m, rows_per_pass(n_j, n_k), n_k, sm_count, device).split;
 }
 
 int launch_tmem_gemm(const LinearArgs& a, cudaStream_t stream) {
@@ -902,6 +920,8 @@ int launch_tmem_gemm(const LinearArgs& a, cudaStream_t stream) {
     return fail(AQ_ERR_INVALID, "the GEMM kernel supports K up to %d, got %d", kMaxNk * kTile,
                 a.n_k * kTile);
   }
+  // Up to 128 rows (one row block here) the weights are the larger operand: a kernel of its own.
+  if (gemm_rows_supported(a.m, a.n_j, a.n_k)) return launch_gemm_rows(a, stream);
   int device = 0;
   int rc = check_cuda(cudaGetDevice(&device), "cudaGetDevice");
   if (rc != AQ_OK) return rc;
@@ -912,7 +932,8 @@ int launch_tmem_gemm(const LinearArgs& a, cudaStream_t stream) {
   alignas(64) CUtensorMap x_map;
   rc = encode_activation_map(&x_map, a.xq, a.m, a.n_k, kBM, 2);
   if (rc != AQ_OK) return rc;
-  Choice choice = choose(a.m, a.n_j, a.n_k, sm_count, device);
+  const int rows_at_once = rows_per_pass(a.n_j, a.n_k);
+  Choice choice = choose(a.m, rows_at_once, a.n_k, sm_count, device);
   if (a.u_metadata != nullptr && choice.split == 1) choice.tn = 4;  // a transformed row needs its 64 columns in one warp
   alignas(64) CUtensorMap out_map;
   rc = encode_result_map(&out_map, a.out, a.out_dtype, a.m, static_cast<int64_t>(a.n_j) * kTile, choice.tn == 4 ? 64 : choice.tn == 3 ? 16 : 32, 32);
@@ -920,7 +941,6 @@ int launch_tmem_gemm(const LinearArgs& a, cudaStream_t stream) {
   const bool dump = a.acc_dump != nullptr;
   const bool fused = !gemm_separate_rounding();
   uint8_t* operand = static_cast<uint8_t*>(a.workspace) + kScratchOffset;
-  const int rows_at_once = rows_per_pass(a.n_j, a.n_k);
   for (int j_base = 0; j_base < a.n_j; j_base += rows_at_once) {
     const int rows = a.n_j - j_base < rows_at_once ? a.n_j - j_base : rows_at_once;
     rc = launch_expand(a.records, a.payload, a.n_k, j_base, rows, choice.tn, operand, stream);

@@ -6,6 +6,7 @@ import numpy as np
 import pytest
 import torch
 
+from alignquant_b200.quantization.exact import metadata_stack
 from oracle import alignquant_oracle as oc
 from tests import helpers
 
@@ -187,3 +188,30 @@ def test_gemm_many_tiles_per_cta_and_column_passes(options, tile, m, n, k):
                                              output_dtype=dtype)
         ext.device_status()
         assert torch.equal(out.cpu(), want.to(dtype))
+
+
+@pytest.mark.parametrize("scale_mode", ["tile", "token"])
+@pytest.mark.parametrize("m", [2, 17, 32, 33, 64, 65, 100, 128])
+@pytest.mark.parametrize("n,k,split", [(64, 64, 1), (192, 320, 1), (320, 1088, 3), (448, 2176, 8), (640, 4096, 0)])
+def test_gemm_of_few_rows_has_the_bits_of_the_other_gemm(options, scale_mode, m, n, k, split):
+    """Up to 128 rows: every row width, an odd number of tile rows, stages that are not full and K ranges of
+    unequal length, against the kernel for many rows with the same K ranges; integer sums against the oracle."""
+    ext = options
+    ext.set_gemm_split(split)
+    weights, tiles, _, xq, a_s, _ = _case(ext, m, n, k, scale_mode, seed=m + n + k)
+    n_j, n_k = n // 64, k // 64
+    u = metadata_stack([-1 if i % 3 == 1 else i + 1 for i in range(n_j)], "cuda")
+    ranges = ext.linear_plan(m, n_j, n_k, schedule="forced_prefill_m64")["splits"]
+    dump = torch.full((m, n_j, n_k, 64), -7, dtype=torch.int32, device="cuda")
+    got = [ext.alignquant_linear_prepared(xq, a_s, weights, meta, schedule="forced_prefill_m64", scale_mode=scale_mode,
+                                          output_dtype=dtype, acc_dump=d)
+           for meta, dtype, d in ((None, torch.float32, dump), (None, torch.bfloat16, None), (u, torch.float16, None))]
+    ext.device_status()
+    assert np.array_equal(dump.cpu().numpy(), oc.tile_accumulators_c(xq.cpu().numpy(), tiles))
+    ext.set_gemm_tile("wide")
+    ext.set_gemm_split(ranges)
+    for have, (meta, dtype) in zip(got, ((None, torch.float32), (None, torch.bfloat16), (u, torch.float16))):
+        want = ext.alignquant_linear_prepared(xq, a_s, weights, meta, schedule="forced_prefill_m64", scale_mode=scale_mode,
+                                              output_dtype=dtype)
+        assert torch.equal(have, want)
+    ext.device_status()
