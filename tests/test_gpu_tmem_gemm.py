@@ -215,3 +215,23 @@ def test_gemm_of_few_rows_has_the_bits_of_the_other_gemm(options, scale_mode, m,
                                               output_dtype=dtype)
         assert torch.equal(have, want)
     ext.device_status()
+
+
+def test_captured_gemms_do_not_share_scratch(ext):
+    """Two graphs captured one after the other (torch captures both on one stream) and replayed at the
+    same time on two streams: each has its own expanded weights."""
+    cases = [_case(ext, 256, 1024, 1024, "token", seed=s) for s in (5, 6)]
+    graphs, results, wants = [], [], []
+    for weights, _, _, xq, a_s, _ in cases:
+        wants.append(ext.alignquant_linear_prepared(xq, a_s, weights, None, scale_mode="token"))
+        torch.cuda.synchronize()
+        graphs.append(torch.cuda.CUDAGraph())
+        with torch.cuda.graph(graphs[-1]):
+            results.append(ext.alignquant_linear_prepared(xq, a_s, weights, None, scale_mode="token"))
+    streams = [torch.cuda.Stream() for _ in graphs]
+    for _ in range(20):
+        for graph, stream in zip(graphs, streams):
+            with torch.cuda.stream(stream):
+                graph.replay()
+    torch.cuda.synchronize()
+    assert all(torch.equal(have, want) for have, want in zip(results, wants))
