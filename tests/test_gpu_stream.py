@@ -39,6 +39,13 @@ def test_repack_image_is_exact(ext, n, k, fraction):
     assert image.size == start + payload.size
 
 
+@pytest.mark.parametrize("fraction", [0.6, 0.0, 1.0])
+@pytest.mark.parametrize("n,k", [(64, 512), (128, 576), (192, 1088), (64, 17024)])
+def test_repack_of_rows_of_several_tile_groups(ext, n, k, fraction):
+    """Full and ragged groups of eight tiles, and more tiles in front of a group than a CTA has threads."""
+    test_repack_image_is_exact(ext, n, k, fraction)
+
+
 @pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
 @pytest.mark.parametrize("m,k", [(1, 64), (5, 192), (16, 3072), (130, 256)])
 def test_token_quantizer_bit_exact(ext, m, k, dtype):
