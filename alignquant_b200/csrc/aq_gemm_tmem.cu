@@ -734,6 +734,7 @@ constexpr int64_t kScratchBytes = 64LL << 20;
 
 // Tile rows per pass, the passes of about one size: the tile width and the K ranges are chosen for a pass.
 int rows_per_pass(int n_j, int n_k) {
+  if (n_k > kMaxNk) return n_j;  // refused at the launch; a scratch of this size holds at least 24 tile rows up to there
   const int64_t most = kScratchBytes / (static_cast<int64_t>(n_k) * kW8TileBytes) / 12 * 12;  // whole CTA tiles of every width
   if (most >= n_j) return n_j;
   const int64_t passes = (n_j + most - 1) / most;
@@ -906,6 +907,7 @@ Choice choose(int64_t m, int n_j, int n_k, int sm_count, int device) {
 }  // namespace
 
 int64_t tmem_gemm_workspace_bytes(int64_t m, int n_j, int n_k) {
+  if (n_k > kMaxNk) return 0;  // the launch says why
   if (gemm_rows_supported(m, n_j, n_k)) return 0;
   const int64_t rows = (rows_per_pass(n_j, n_k) + 11) / 12 * 12;
   return kScratchOffset + rows * n_k * kW8TileBytes;

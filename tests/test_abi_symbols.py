@@ -6,6 +6,8 @@ import ctypes
 import re
 from pathlib import Path
 
+import pytest
+
 from alignquant_b200 import _lib
 
 HEADER = Path(__file__).resolve().parents[1] / "include" / "alignquant_b200.h"
@@ -32,6 +34,20 @@ def test_pure_host_entry_points():
     assert lib.aq_prepared_bytes(2, 3, 4, 1) < 0 and "t4 + t8" in _lib.last_error()
     assert lib.aq_linear_workspace_bytes(0, 1, 1, 0, 0) < 0
     assert lib.aq_linear_workspace_bytes(64, 4, 4, 0, 4) == 0  # explicit splits: cluster kernel, no scratch
+
+
+@pytest.mark.parametrize("n_k", [513, 1365, 1366, 20000])
+@pytest.mark.parametrize("m,schedule", [(33, 0), (128, 0), (129, 0), (4096, 0), (2, 3), (129, 3)])
+def test_k_above_the_gemm_limit_is_refused_with_a_message(m, schedule, n_k):
+    """Size and plan queries answer for any K, and the call says what its limit is (no launch, so no GPU)."""
+    lib = _lib.load()
+    assert lib.aq_linear_workspace_bytes(m, 4, n_k, schedule, 0) == 0
+    kernel, splits, workers = (ctypes.c_int32() for _ in range(3))
+    assert lib.aq_linear_plan(m, 4, n_k, schedule, 0, *(ctypes.addressof(v) for v in (kernel, splits, workers))) == 0
+    assert kernel.value == 1 and splits.value >= 1
+    at = 1 << 20  # never read
+    assert lib.aq_linear(at, at, _lib.AQ_SCALE_TOKEN, m, at, 4, n_k, None, schedule, 0, _lib.AQ_F32, at, None, 0, None, None) == -1
+    assert "K up to 32768" in _lib.last_error()
 
 
 def test_options_are_validated_and_read_back():
