@@ -185,61 +185,39 @@ __device__ __forceinline__ void store_out<__nv_bfloat16>(__nv_bfloat16* out, int
   out[index] = __float2bfloat16_rn(value);
 }
 
-// 64-point unnormalised Walsh-Hadamard transforms of kRows rows held by a warp:
-// lane l owns elements l (low) and l + 32 (high) of each.
-template <int kRows>
-__device__ __forceinline__ void fwht64_warp(double (&low)[kRows], double (&high)[kRows], int lane) {
+// 64-point unnormalised Walsh-Hadamard transform of one row held by a warp:
+// lane l owns elements l (low) and l + 32 (high).
+__device__ __forceinline__ void fwht64_warp(double& low, double& high, int lane) {
 #pragma unroll
   for (int stride = 1; stride < 32; stride <<= 1) {
-#pragma unroll
-    for (int r = 0; r < kRows; ++r) {
-      const double low_peer = __shfl_xor_sync(0xffffffffu, low[r], stride);
-      const double high_peer = __shfl_xor_sync(0xffffffffu, high[r], stride);
-      low[r] = (lane & stride) ? low_peer - low[r] : low[r] + low_peer;
-      high[r] = (lane & stride) ? high_peer - high[r] : high[r] + high_peer;
-    }
+    const double low_peer = __shfl_xor_sync(0xffffffffu, low, stride);
+    const double high_peer = __shfl_xor_sync(0xffffffffu, high, stride);
+    low = (lane & stride) ? low_peer - low : low + low_peer;
+    high = (lane & stride) ? high_peer - high : high + high_peer;
   }
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) {
-    const double a = low[r], b = high[r];
-    low[r] = a + b;
-    high[r] = a - b;
-  }
+  const double a = low, b = high;
+  low = a + b;
+  high = a - b;
 }
 
-// Inverse output transform of kRows 64-column rows held by a warp (lane l owns columns
+// Inverse output transform of one 64-column row held by a warp (lane l owns columns
 // l and l + 32): out[r] = left[r] * ((acc * right) H)[perm[r]] / 8, evaluated in FP64
 // (alignquant/kernels/cuda/linear.cu:404-430, 1003-1036).  `meta` points at the
-// [4][64] int32 rows (mode, permutation, left sign, right sign) of the tile.  A row is a chain of some
-// twenty dependent shuffles; where a warp has several rows, they are worth doing together.
-template <int kRows>
-__device__ __forceinline__ void inverse_u_rows(float (&lo)[kRows], float (&hi)[kRows], const int32_t* meta, int lane) {
-  double dl[kRows], dh[kRows];
-  const double right_lo = static_cast<double>(meta[3 * kTile + lane]), right_hi = static_cast<double>(meta[3 * kTile + lane + 32]);
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) {
-    dl[r] = static_cast<double>(lo[r]) * right_lo;
-    dh[r] = static_cast<double>(hi[r]) * right_hi;
-  }
+// [4][64] int32 rows (mode, permutation, left sign, right sign) of the tile.
+__device__ __forceinline__ void inverse_u_row(float& lo, float& hi, const int32_t* meta, int lane) {
+  double dl = static_cast<double>(lo) * static_cast<double>(meta[3 * kTile + lane]);
+  double dh = static_cast<double>(hi) * static_cast<double>(meta[3 * kTile + lane + 32]);
   fwht64_warp(dl, dh, lane);
   const int t_lo = meta[kTile + lane];
   const int t_hi = meta[kTile + lane + 32];
-  const double left_lo = static_cast<double>(meta[2 * kTile + lane]), left_hi = static_cast<double>(meta[2 * kTile + lane + 32]);
-#pragma unroll
-  for (int r = 0; r < kRows; ++r) {
-    const double lo_from_l = __shfl_sync(0xffffffffu, dl[r], t_lo & 31);
-    const double lo_from_h = __shfl_sync(0xffffffffu, dh[r], t_lo & 31);
-    const double hi_from_l = __shfl_sync(0xffffffffu, dl[r], t_hi & 31);
-    const double hi_from_h = __shfl_sync(0xffffffffu, dh[r], t_hi & 31);
-    lo[r] = static_cast<float>((t_lo < 32 ? lo_from_l : lo_from_h) * left_lo * 0.125);
-    hi[r] = static_cast<float>((t_hi < 32 ? hi_from_l : hi_from_h) * left_hi * 0.125);
-  }
-}
-__device__ __forceinline__ void inverse_u_row(float& lo, float& hi, const int32_t* meta, int lane) {
-  float l[1] = {lo}, h[1] = {hi};
-  inverse_u_rows(l, h, meta, lane);
-  lo = l[0];
-  hi = h[0];
+  const double lo_from_l = __shfl_sync(0xffffffffu, dl, t_lo & 31);
+  const double lo_from_h = __shfl_sync(0xffffffffu, dh, t_lo & 31);
+  const double hi_from_l = __shfl_sync(0xffffffffu, dl, t_hi & 31);
+  const double hi_from_h = __shfl_sync(0xffffffffu, dh, t_hi & 31);
+  lo = static_cast<float>((t_lo < 32 ? lo_from_l : lo_from_h) *
+                          static_cast<double>(meta[2 * kTile + lane]) * 0.125);
+  hi = static_cast<float>((t_hi < 32 ? hi_from_l : hi_from_h) *
+                          static_cast<double>(meta[2 * kTile + lane + 32]) * 0.125);
 }
 
 #endif  // __CUDACC__

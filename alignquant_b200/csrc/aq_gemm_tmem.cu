@@ -77,8 +77,6 @@ constexpr int kScaleSlots = 16;     // K steps whose scales are kept: more than 
 constexpr int kScaleRow = 12;       // floats per step: TN <= 4 weight scales, then eight activation scales (tile mode)
 constexpr int kTurnRows = 15;       // rows a drain warp turns through shared memory at a time (output transform)
 constexpr int kTurnFloats = 65;     // floats per turned row
-constexpr int kTurnTogether = 3;    // turned rows transformed together
-static_assert(kTurnRows % kTurnTogether == 0 && kTurnRows * 65 * 4 <= 4096, "turned rows");
 constexpr int kTurnBytes = 4096;    // shared memory in which a drain warp turns its results
 
 // TN = weight tile rows (64 columns each) of the CTA tile.  A stage of the ring holds two K steps:
@@ -278,9 +276,7 @@ __device__ __forceinline__ void dump16(const GemmParams& p, int64_t row, int j, 
   }
 }
 
-// kU: with output transforms.  Wide tiles without them are an instantiation of its own: the transform's registers
-// would cost the drain loop spills.
-template <int TN, bool kDump, bool kFused, bool kU>
+template <int TN, bool kDump, bool kFused>
 __global__ void __launch_bounds__(kThreads, 1)
 tmem_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap out_map, const GemmParams p) {
   using S = Layout<TN>;
@@ -572,10 +568,10 @@ tmem_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
       } else if (ok && j < p.n_j) {
         const int64_t n_cols = p.row_stride;
         const int32_t* meta = p.u_metadata ? p.u_metadata + static_cast<int64_t>(j) * 4 * kTile : nullptr;
-        if (TN != 4 || !kU || meta == nullptr || meta[0] == 0) {
+        if (TN != 4 || meta == nullptr || meta[0] == 0) {
           if (row0 < p.m) store_rows<kWarpCols>(&out_map, p.out_dtype, turn + warp * kTurnBytes, static_cast<int>(row0), j * kTile + tile_col,
                                                 static_cast<int>(p.row_stride), lane, acc);
-        } else if constexpr (TN == 4 && kU) {
+        } else if constexpr (TN == 4) {
           // Output transform: a few rows at a time change from one lane per row to two columns
           // per lane (the stage ring already belongs to the next output tile).
           float* region = reinterpret_cast<float*>(turn + warp * kTurnBytes);
@@ -588,26 +584,16 @@ tmem_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
               for (int c = 0; c < kWarpCols / 2; ++c) unpack2(acc[c], dst[2 * c], dst[2 * c + 1]);
             }
             __syncwarp();
-            // three rows together: their chains of shuffles overlap (five spill in the drain loop).  Rows past
-            // those turned are stale and not stored.
 #pragma unroll 1
-            for (int r = 0; r < kTurnRows && r0 + r < 32 && row0 + r0 + r < p.m; r += kTurnTogether) {
-              float lo[kTurnTogether], hi[kTurnTogether];
-#pragma unroll
-              for (int h = 0; h < kTurnTogether; ++h) {
-                lo[h] = region[(r + h) * kTurnFloats + lane];
-                hi[h] = region[(r + h) * kTurnFloats + lane + 32];
-              }
-              inverse_u_rows(lo, hi, meta, lane);
-#pragma unroll
-              for (int h = 0; h < kTurnTogether; ++h) {
-                const int64_t gr = row0 + r0 + r + h;
-                if (r0 + r + h < 32 && gr < p.m) {
-                  const int64_t o = gr * n_cols + static_cast<int64_t>(j) * kTile + lane;
-                  store_any(p.out, p.out_dtype, o, lo[h]);
-                  store_any(p.out, p.out_dtype, o + 32, hi[h]);
-                }
-              }
+            for (int r = 0; r < kTurnRows && r0 + r < 32; ++r) {
+              const int64_t gr = row0 + r0 + r;
+              if (gr >= p.m) break;
+              float lo = region[r * kTurnFloats + lane];
+              float hi = region[r * kTurnFloats + lane + 32];
+              inverse_u_row(lo, hi, meta, lane);
+              const int64_t o = gr * n_cols + static_cast<int64_t>(j) * kTile + lane;
+              store_any(p.out, p.out_dtype, o, lo);
+              store_any(p.out, p.out_dtype, o + 32, hi);
             }
           }
         }
@@ -661,7 +647,7 @@ tmem_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
         }
         const int j = p.j_base + nb * TN + tl;
         const int32_t* meta = p.u_metadata ? p.u_metadata + static_cast<int64_t>(j) * 4 * kTile : nullptr;
-        if (kU && meta != nullptr && meta[0] != 0) inverse_u_row(lo, hi, meta, lane);
+        if (meta != nullptr && meta[0] != 0) inverse_u_row(lo, hi, meta, lane);
         const int64_t o = (m0 + row) * n_cols + static_cast<int64_t>(j) * kTile + lane;
         store_any(p.out, p.out_dtype, o, lo);
         store_any(p.out, p.out_dtype, o + 32, hi);
@@ -760,15 +746,11 @@ int set_shared_memory(int device) {
   static std::once_flag once[64];
   cudaError_t attr_status = cudaSuccess;
   std::call_once(once[device & 63], [&] {
-    const void* kernels[8] = {
-        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, false, true>),
-        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, true, true>),
-        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, true, false, true>),
-        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, true, true, true>),
-        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, false, TN != 4>),
-        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, true, TN != 4>),
-        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, true, false, TN != 4>),
-        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, true, true, TN != 4>)};
+    const void* kernels[4] = {
+        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, false>),
+        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, true>),
+        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, true, false>),
+        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, true, true>)};
     for (const void* kernel : kernels) {
       if (attr_status == cudaSuccess) {
         attr_status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<TN>::kSmemBytes);
@@ -800,7 +782,7 @@ int resident_clusters(int split, int device) {
     config.attrs = attr;
     config.numAttrs = 1;
     if (set_shared_memory<TN>(device) != AQ_OK ||
-        cudaOccupancyMaxActiveClusters(&clusters, reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, true, true>), &config) != cudaSuccess) {
+        cudaOccupancyMaxActiveClusters(&clusters, reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, true>), &config) != cudaSuccess) {
       (void)cudaGetLastError();
       clusters = 0;
     }
@@ -831,12 +813,14 @@ int launch_shape(const CUtensorMap& x_map, const CUtensorMap& out_map, const Gem
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
   config.numAttrs = use_dependent_launch() ? 2 : 1;
-  const bool u = TN != 4 || p.u_metadata != nullptr;
-  const auto kernel = dump ? (fused ? (u ? tmem_gemm_kernel<TN, true, true, true> : tmem_gemm_kernel<TN, true, true, TN != 4>)
-                                    : (u ? tmem_gemm_kernel<TN, true, false, true> : tmem_gemm_kernel<TN, true, false, TN != 4>))
-                           : (fused ? (u ? tmem_gemm_kernel<TN, false, true, true> : tmem_gemm_kernel<TN, false, true, TN != 4>)
-                                    : (u ? tmem_gemm_kernel<TN, false, false, true> : tmem_gemm_kernel<TN, false, false, TN != 4>));
-  const cudaError_t status = cudaLaunchKernelEx(&config, kernel, x_map, out_map, p);
+  cudaError_t status;
+  if (dump) {
+    status = fused ? cudaLaunchKernelEx(&config, tmem_gemm_kernel<TN, true, true>, x_map, out_map, p)
+                   : cudaLaunchKernelEx(&config, tmem_gemm_kernel<TN, true, false>, x_map, out_map, p);
+  } else {
+    status = fused ? cudaLaunchKernelEx(&config, tmem_gemm_kernel<TN, false, true>, x_map, out_map, p)
+                   : cudaLaunchKernelEx(&config, tmem_gemm_kernel<TN, false, false>, x_map, out_map, p);
+  }
   return check_cuda(status, "tensor-memory GEMM launch");
 }
 
