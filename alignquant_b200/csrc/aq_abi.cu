@@ -245,7 +245,7 @@ int64_t aq_linear_workspace_bytes(int64_t m, int32_t n_j, int32_t n_k, int sched
   }
   switch (choose_kernel(m, n_j, n_k, schedule, decode_splits)) {
     case 1:
-      return tmem_gemm_workspace_bytes(m, n_j, n_k);
+      return plan_gemm(m, n_j, n_k).workspace_bytes;
     case 2:
       return decode_workspace_bytes(m, n_j, n_k);
     default:
@@ -357,12 +357,13 @@ static int linear_impl(const int8_t* xq, const float* act_scales, int scale_mode
     const int split = decode_splits != 0 ? decode_splits : stream_auto_split(m, n_j, n_k);
     return launch_stream_linear(a, split, s);
   }
-  const int64_t need = kernel == 2 ? decode_workspace_bytes(m, n_j, n_k) : tmem_gemm_workspace_bytes(m, n_j, n_k);
+  const GemmPlan plan = kernel == 1 ? plan_gemm(m, n_j, n_k) : GemmPlan{};
+  const int64_t need = kernel == 2 ? decode_workspace_bytes(m, n_j, n_k) : plan.workspace_bytes;
   if (need > 0 && (workspace == nullptr || workspace_bytes < need || !aligned(workspace, 256))) {
     return fail(AQ_ERR_WORKSPACE, "aq_linear needs a 256-byte aligned workspace of %lld bytes",
                 static_cast<long long>(need));
   }
-  return kernel == 2 ? launch_decode_linear(a, s) : launch_tmem_gemm(a, s);
+  return kernel == 2 ? launch_decode_linear(a, s) : launch_tmem_gemm(a, plan, s);
 }
 
 
@@ -488,7 +489,7 @@ int aq_linear_plan(int64_t m, int32_t n_j, int32_t n_k, int schedule, int decode
     while (s > n_k) s /= 2;
     *splits = s;  // the launcher may raise it further for very long K; see aq_stream.cu
   } else if (k == 1) {
-    *splits = tmem_gemm_split(m, n_j, n_k);
+    *splits = plan_gemm(m, n_j, n_k).split;
   } else if (k == 2) {
     *splits = decode_ctas(n_j, n_k);
     *workers = 16;

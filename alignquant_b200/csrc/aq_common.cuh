@@ -125,16 +125,23 @@ int take_decode_status();
 int launch_decode_linear_static(const LinearArgs& a, cudaStream_t stream);
 int64_t decode_static_scratch_bytes();
 
-// Tensor-memory GEMM (tcgen05) for large m.
-int launch_tmem_gemm(const LinearArgs& a, cudaStream_t stream);
-int64_t tmem_gemm_workspace_bytes(int64_t m, int n_j, int n_k);
-int tmem_gemm_split(int64_t m, int n_j, int n_k);  // K ranges (cluster size) the GEMM will use
+// Tensor-memory GEMM (tcgen05) for large m.  The process-wide options are read once, when a call is planned: what
+// its workspace was checked against is what is launched, whatever another thread sets meanwhile.
+struct GemmPlan {
+  bool few_rows;            // gemm_rows_kernel; else the expansion of the weights and tmem_gemm_kernel
+  bool fused;               // one rounding per tile (AQ_OPT_GEMM_ROUNDING)
+  int tn;                   // tile rows of a CTA tile                 (not few_rows)
+  int rows_per_pass;        // tile rows expanded at a time            (not few_rows)
+  int split;                // K ranges (cluster size)
+  int64_t workspace_bytes;  // 0: none
+};
+GemmPlan plan_gemm(int64_t m, int n_j, int n_k);
+int launch_tmem_gemm(const LinearArgs& a, const GemmPlan& plan, cudaStream_t stream);
 
-// GEMM for up to 128 rows that reads the packed weights once (what launch_tmem_gemm runs where it applies).
-bool gemm_rows_supported(int64_t m, int n_j, int n_k);
-int gemm_rows_split(int64_t m, int n_j, int n_k, double* cost);  // K ranges, and the modelled SM cycles
-double tmem_gemm_cost(int64_t m, int n_j, int n_k);  // the same for the GEMM with expanded weights
-int launch_gemm_rows(const LinearArgs& a, cudaStream_t stream);
+// GEMM for up to 128 rows that reads the packed weights once: K ranges (`forced`: AQ_OPT_GEMM_SPLIT) and their modelled
+// SM cycles, and the launch.
+int gemm_rows_split(int64_t m, int n_j, int n_k, int forced, double* cost);
+int launch_gemm_rows(const LinearArgs& a, int split, cudaStream_t stream);
 int take_gemm_rows_status();
 
 // Rate of back-to-back tcgen05.mma kind::i8 on all SMs (measurement aid; synchronises).

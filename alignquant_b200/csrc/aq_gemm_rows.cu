@@ -559,9 +559,8 @@ int resident_clusters(const Shape& shape, int split, int device) {
 
 // K ranges and their cost by a model in SM cycles: a K step of two tiles (measured 520, 650 and 1060 for 32, 64
 // and 128 rows), what a CTA costs beside its steps, the exchange; clusters in waves.
-// AQ_OPT_GEMM_SPLIT forces a number.
-int gemm_rows_split(int64_t m, int n_j, int n_k, double* cost) {
-  const int forced = gemm_split_option();
+// `forced` (AQ_OPT_GEMM_SPLIT) >= 1: that number.
+int gemm_rows_split(int64_t m, int n_j, int n_k, int forced, double* cost) {
   const int pairs = (n_j + 1) / 2;
   const double step = m <= 32 ? 520.0 : m <= 64 ? 650.0 : 1060.0;
   int device = 0;
@@ -585,18 +584,7 @@ int gemm_rows_split(int64_t m, int n_j, int n_k, double* cost) {
   return best;
 }
 
-// Where the packed weights' single pass costs less than their expansion and the GEMM for many rows (both
-// by their models).  Measured (us, this kernel / the other): 48 rows 34816 x 5120 61 / 110, 5120 x 17408 34 / 82, 3072 x
-// 3072 8.9 / 12.9, 19456 x 2560 (152 CTAs: a second wave of four) 36 / 33; 75 rows 16384 x 3072 31 / 28.5.
-bool gemm_rows_supported(int64_t m, int n_j, int n_k) {
-  if (m > 128 || gemm_separate_rounding() || gemm_tile_option() != AQ_GEMM_TILE_AUTO) return false;
-  if (gemm_split_option() >= 1) return true;
-  double cost = 0.0;
-  gemm_rows_split(m, n_j, n_k, &cost);
-  return cost < tmem_gemm_cost(m, n_j, n_k);
-}
-
-int launch_gemm_rows(const LinearArgs& a, cudaStream_t stream) {
+int launch_gemm_rows(const LinearArgs& a, int split, cudaStream_t stream) {
   int device = 0;
   int rc = check_cuda(cudaGetDevice(&device), "cudaGetDevice");
   if (rc != AQ_OK) return rc;
@@ -619,7 +607,7 @@ int launch_gemm_rows(const LinearArgs& a, cudaStream_t stream) {
   p.out_dtype = a.out_dtype;
   cudaLaunchConfig_t config = {};
   cudaLaunchAttribute attr[2];
-  fill_config(&config, attr, shape, (a.n_j + 1) / 2, gemm_rows_split(a.m, a.n_j, a.n_k, nullptr));
+  fill_config(&config, attr, shape, (a.n_j + 1) / 2, split);
   config.stream = stream;
   if (use_dependent_launch()) {
     attr[1].id = cudaLaunchAttributeProgrammaticStreamSerialization;

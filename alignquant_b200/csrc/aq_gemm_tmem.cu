@@ -854,9 +854,7 @@ struct Choice {
 // 69 us against 77); K ranges only pay for a few row blocks (128 x 5120 x 3072: 16 us against 21).
 // `n_j`: tile rows of a pass (with the whole layer's, 34816 x 5120 at 48 rows ran three passes of 48 CTAs).
 // AQ_OPT_GEMM_TILE and AQ_OPT_GEMM_SPLIT force a choice.
-Choice choose(int64_t m, int n_j, int n_k, int sm_count, int device) {
-  const int forced_tile = gemm_tile_option();
-  const int forced_split = gemm_split_option();
+Choice choose(int64_t m, int n_j, int n_k, int forced_tile, int forced_split, int sm_count, int device) {
   const int64_t m_blocks = (m + kBM - 1) / kBM;
   static const double kStep[5] = {0, 0, 527, 730, 850};
   static const double kHandOver[5] = {0, 0, 1400, 3000, 1800};
@@ -890,40 +888,45 @@ Choice choose(int64_t m, int n_j, int n_k, int sm_count, int device) {
 
 }  // namespace
 
-int64_t tmem_gemm_workspace_bytes(int64_t m, int n_j, int n_k) {
-  if (n_k > kMaxNk) return 0;  // the launch says why
-  if (gemm_rows_supported(m, n_j, n_k)) return 0;
-  const int64_t rows = (rows_per_pass(n_j, n_k) + 11) / 12 * 12;
-  return kScratchOffset + rows * n_k * kW8TileBytes;
-}
-
-// Expansion (2.1 cycles per tile, measured: 14 us for 12288 tiles) and GEMM, pass by pass.
-double tmem_gemm_cost(int64_t m, int n_j, int n_k) {
+// Up to 128 rows the kernel that reads the packed weights once, where that pass costs less than their expansion and
+// the GEMM for many rows, both by their models (expansion: 2.1 cycles per tile, measured: 14 us for 12288 tiles).
+// Measured (us, gemm_rows_kernel / the other): 48 rows 34816 x 5120 61 / 110, 5120 x 17408 34 / 82, 3072 x 3072 8.9 /
+// 12.9, 19456 x 2560 (152 CTAs: a second wave of four) 36 / 33; 75 rows 16384 x 3072 31 / 28.5.
+GemmPlan plan_gemm(int64_t m, int n_j, int n_k) {
+  const int forced_tile = gemm_tile_option();
+  const int forced_split = gemm_split_option();
   int sm_count = 148;
   if (device_sm_count(&sm_count) != AQ_OK) sm_count = 148;
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess) device = 0;
-  const int rows = rows_per_pass(n_j, n_k);
-  const int passes = (n_j + rows - 1) / rows;
-  return passes * choose(m, rows, n_k, sm_count, device).cost + 2.1 * static_cast<double>(n_j) * n_k + 2000.0;
+  GemmPlan plan = {};
+  plan.fused = !gemm_separate_rounding();
+  plan.rows_per_pass = rows_per_pass(n_j, n_k);
+  const Choice choice = choose(m, plan.rows_per_pass, n_k, forced_tile, forced_split, sm_count, device);
+  plan.tn = choice.tn;
+  plan.split = choice.split;
+  if (n_k > kMaxNk) return plan;  // the launch says why
+  if (m <= kBM && plan.fused && forced_tile == AQ_GEMM_TILE_AUTO) {
+    const int passes = (n_j + plan.rows_per_pass - 1) / plan.rows_per_pass;
+    const double cost = passes * choice.cost + 2.1 * static_cast<double>(n_j) * n_k + 2000.0;
+    double rows_cost = 0.0;
+    const int rows_split = gemm_rows_split(m, n_j, n_k, forced_split, &rows_cost);
+    if (forced_split >= 1 || rows_cost < cost) {
+      plan.few_rows = true;
+      plan.split = rows_split;
+      return plan;
+    }
+  }
+  plan.workspace_bytes = kScratchOffset + static_cast<int64_t>((plan.rows_per_pass + 11) / 12 * 12) * n_k * kW8TileBytes;
+  return plan;
 }
 
-int tmem_gemm_split(int64_t m, int n_j, int n_k) {
-  if (gemm_rows_supported(m, n_j, n_k)) return gemm_rows_split(m, n_j, n_k, nullptr);
-  int sm_count = 148;
-  if (device_sm_count(&sm_count) != AQ_OK) sm_count = 148;
-  int device = 0;
-  if (cudaGetDevice(&device) != cudaSuccess) device = 0;
-  return choose(m, rows_per_pass(n_j, n_k), n_k, sm_count, device).split;
-}
-
-int launch_tmem_gemm(const LinearArgs& a, cudaStream_t stream) {
+int launch_tmem_gemm(const LinearArgs& a, const GemmPlan& plan, cudaStream_t stream) {
   if (a.n_k > kMaxNk) {
     return fail(AQ_ERR_INVALID, "the GEMM kernel supports K up to %d, got %d", kMaxNk * kTile,
                 a.n_k * kTile);
   }
-  // Up to 128 rows (one row block here) the weights are the larger operand: a kernel of its own.
-  if (gemm_rows_supported(a.m, a.n_j, a.n_k)) return launch_gemm_rows(a, stream);
+  if (plan.few_rows) return launch_gemm_rows(a, plan.split, stream);
   int device = 0;
   int rc = check_cuda(cudaGetDevice(&device), "cudaGetDevice");
   if (rc != AQ_OK) return rc;
@@ -934,18 +937,16 @@ int launch_tmem_gemm(const LinearArgs& a, cudaStream_t stream) {
   alignas(64) CUtensorMap x_map;
   rc = encode_activation_map(&x_map, a.xq, a.m, a.n_k, kBM, 2);
   if (rc != AQ_OK) return rc;
-  const int rows_at_once = rows_per_pass(a.n_j, a.n_k);
-  Choice choice = choose(a.m, rows_at_once, a.n_k, sm_count, device);
-  if (a.u_metadata != nullptr && choice.split == 1) choice.tn = 4;  // a transformed row needs its 64 columns in one warp
+  const int rows_at_once = plan.rows_per_pass;
+  const int tn = a.u_metadata != nullptr && plan.split == 1 ? 4 : plan.tn;  // a transformed row needs its 64 columns in one warp
   alignas(64) CUtensorMap out_map;
-  rc = encode_result_map(&out_map, a.out, a.out_dtype, a.m, static_cast<int64_t>(a.n_j) * kTile, choice.tn == 4 ? 64 : choice.tn == 3 ? 16 : 32, 32);
+  rc = encode_result_map(&out_map, a.out, a.out_dtype, a.m, static_cast<int64_t>(a.n_j) * kTile, tn == 4 ? 64 : tn == 3 ? 16 : 32, 32);
   if (rc != AQ_OK) return rc;
   const bool dump = a.acc_dump != nullptr;
-  const bool fused = !gemm_separate_rounding();
   uint8_t* operand = static_cast<uint8_t*>(a.workspace) + kScratchOffset;
   for (int j_base = 0; j_base < a.n_j; j_base += rows_at_once) {
     const int rows = a.n_j - j_base < rows_at_once ? a.n_j - j_base : rows_at_once;
-    rc = launch_expand(a.records, a.payload, a.n_k, j_base, rows, choice.tn, operand, stream);
+    rc = launch_expand(a.records, a.payload, a.n_k, j_base, rows, tn, operand, stream);
     if (rc != AQ_OK) return rc;
     GemmParams p;
     p.act_scales = a.act_scales;
@@ -963,12 +964,12 @@ int launch_tmem_gemm(const LinearArgs& a, cudaStream_t stream) {
     p.scale_mode = a.scale_mode;
     p.out_dtype = a.out_dtype;
     p.m_blocks = static_cast<int>((a.m + kBM - 1) / kBM);
-    p.n_blocks = (rows + choice.tn - 1) / choice.tn;
+    p.n_blocks = (rows + tn - 1) / tn;
     p.band_magic = static_cast<uint32_t>((1ULL << 32) / (static_cast<uint64_t>(p.n_blocks) * 16));
     if (static_cast<int64_t>(p.m_blocks) * p.n_blocks >= (1LL << 31) / 16) return fail(AQ_ERR_INVALID, "the GEMM kernel supports fewer output tiles");
-    rc = choice.tn == 4   ? launch_shape<4>(x_map, out_map, p, dump, fused, choice.split, sm_count, device, stream)
-         : choice.tn == 3 ? launch_shape<3>(x_map, out_map, p, dump, fused, choice.split, sm_count, device, stream)
-                          : launch_shape<2>(x_map, out_map, p, dump, fused, choice.split, sm_count, device, stream);
+    rc = tn == 4   ? launch_shape<4>(x_map, out_map, p, dump, plan.fused, plan.split, sm_count, device, stream)
+         : tn == 3 ? launch_shape<3>(x_map, out_map, p, dump, plan.fused, plan.split, sm_count, device, stream)
+                          : launch_shape<2>(x_map, out_map, p, dump, plan.fused, plan.split, sm_count, device, stream);
     if (rc != AQ_OK) return rc;
   }
   return AQ_OK;

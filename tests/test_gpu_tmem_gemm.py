@@ -2,10 +2,13 @@
 
 from __future__ import annotations
 
+import threading
+
 import numpy as np
 import pytest
 import torch
 
+from alignquant_b200 import _lib
 from alignquant_b200.quantization.exact import metadata_stack
 from oracle import alignquant_oracle as oc
 from tests import helpers
@@ -235,3 +238,35 @@ def test_captured_gemms_do_not_share_scratch(ext):
                 graph.replay()
     torch.cuda.synchronize()
     assert all(torch.equal(have, want) for have, want in zip(results, wants))
+
+
+def test_options_set_by_another_thread_meet_whole_calls(options):
+    """A call is planned once: with an option changing all the time, each call without a workspace runs the
+    kernel that needs none or is refused, and never launches what its workspace was not checked for."""
+    ext = options
+    ext.set_gemm_split(1)
+    m, n, k = 100, 640, 1024
+    weights, _, _, xq, a_s, _ = _case(ext, m, n, k, "token", seed=12)
+    want = ext.alignquant_linear_prepared(xq, a_s, weights, None, scale_mode="token")
+    lib, stop = _lib.load(), threading.Event()
+
+    def toggle():
+        while not stop.is_set():
+            for tile in (_lib.GEMM_TILES["wide"], _lib.GEMM_TILES["auto"]):
+                lib.aq_set_option(_lib.AQ_OPT_GEMM_TILE, tile)
+
+    thread = threading.Thread(target=toggle)
+    thread.start()
+    try:
+        seen = {0: 0, -3: 0}
+        for _ in range(2000):
+            out = torch.zeros_like(want)
+            status = lib.aq_linear(xq.data_ptr(), a_s.data_ptr(), _lib.AQ_SCALE_TOKEN, m, weights.image.data_ptr(), n // 64, k // 64,
+                                   None, 0, 0, _lib.AQ_F32, out.data_ptr(), None, 0, None, torch.cuda.current_stream().cuda_stream)
+            seen[status] += 1  # 0, or AQ_ERR_WORKSPACE
+            assert status != 0 or torch.equal(out, want)
+    finally:
+        stop.set()
+        thread.join()
+    ext.device_status()
+    assert seen[0] > 0
