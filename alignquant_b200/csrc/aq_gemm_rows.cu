@@ -315,6 +315,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap x_map, const RowsParams p) 
     grid_dependency_wait();  // the activation scales come from the preceding kernel, and it may read what is stored here
     constexpr int kRowGroups = kCols / 16;  // 16-row groups of the warp, one scale each per step under tile scales
     float g_next[kToken ? 1 : kSub][kRowGroups];
+    // Ordinary loads, as for all that the preceding kernel writes: it may still be writing while this one is resident,
+    // and the read-only path does not see that (stale scales at 128 x 3072 x 3072).
     auto group_scales = [&](int at) {
       if constexpr (!kToken) {
 #pragma unroll
@@ -323,7 +325,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap x_map, const RowsParams p) 
           for (int g = 0; g < kRowGroups; ++g) {
             const int row_group = group * kRowGroups + g;
             g_next[s][g] = at + s < steps && row_group * 16 < p.m
-                               ? __ldg(p.act_scales + static_cast<int64_t>(row_group) * n_k + k_begin + at + s)
+                               ? p.act_scales[static_cast<int64_t>(row_group) * n_k + k_begin + at + s]
                                : 0.0f;
           }
         }

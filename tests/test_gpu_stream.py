@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 import torch
 
+from alignquant_b200.synthetic import synthetic_module_tensors
 from oracle import alignquant_oracle as oc
 from tests import helpers
 
@@ -475,3 +476,42 @@ def test_argument_errors_raise(ext):
     with pytest.raises(RuntimeError, match="selected payload count mismatch"):
         ext.prepare_weights(t["state_bits"], t["w4_payload"], t["w4_scales"], t["w8_payload"], t["w8_scales"],
                             t["w4_row_offsets"], t["w8_row_offsets"], n_k=2)
+
+
+@pytest.mark.parametrize("scale_mode", ["token", "tile", "norm"])
+@pytest.mark.parametrize("n", [512, 3072])
+@pytest.mark.parametrize("m", [1, 4, 16, 24, 32, 48, 128, 300, 1024])
+def test_chained_calls_read_what_the_call_before_has_just_written(ext, scale_mode, m, n):
+    """Rows, codes and scales in buffers that every call of a captured chain writes anew: under dependent launch a kernel
+    is resident while the ones before it still read the old content and write the new one."""
+    t = synthetic_module_tensors(n, n, 7)
+    weights = ext.prepare_weights(*(t[name] for name in ("state_bits", "w4_payload", "w4_scales", "w8_payload", "w8_scales",
+                                                         "w4_row_offsets", "w8_row_offsets")), n_k=n // 64)
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    first = torch.randn(m, n, generator=gen, device="cuda").to(torch.bfloat16)
+    norm = (1.0 + 0.1 * torch.randn(n, generator=gen, device="cuda")).to(torch.bfloat16)
+    x = first.clone()
+    mode = "tile" if scale_mode == "tile" else "token"
+    codes = ext.alignquant_activation_quantize_cuda(x, None, scale_mode=mode)
+
+    def step():
+        if scale_mode == "norm":
+            ext.alignquant_rmsnorm_quantize_cuda(x, norm, 1e-6, out=codes)
+        else:
+            ext.alignquant_activation_quantize_cuda(x, None, scale_mode=mode, out=codes)
+        ext.alignquant_linear_prepared(*codes, weights, None, scale_mode=mode, output_dtype=torch.bfloat16, out=x)
+
+    for _ in range(6):
+        step()
+        torch.cuda.synchronize()
+    want = x.clone()
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        x.copy_(first)
+        for _ in range(6):
+            step()
+    for _ in range(20):
+        graph.replay()
+        torch.cuda.synchronize()
+        assert torch.equal(x, want)
+    ext.device_status()
