@@ -305,7 +305,7 @@ __global__ void __launch_bounds__(32 * WARPS, NG == 1 ? 3 : 2) direct_decode_ker
       float amax = 0.0f;
       for (int v = threadIdx.x; v < vectors_per_row; v += kThreads) {
         float f[8];
-        unpack8(__ldg(raw_global + static_cast<int64_t>(r) * vectors_per_row + v), raw_bf16, f);
+        unpack8(load_global_v4(raw_global + static_cast<int64_t>(r) * vectors_per_row + v), raw_bf16, f);
 #pragma unroll
         for (int i = 0; i < 8; ++i) amax = fmaxf(amax, fabsf(f[i]));
       }
@@ -330,7 +330,7 @@ __global__ void __launch_bounds__(32 * WARPS, NG == 1 ? 3 : 2) direct_decode_ker
       const float inv_scale = __fdiv_rn(1.0f, scale);
       for (int v = threadIdx.x; v < vectors_per_row; v += kThreads) {
         float f[8];
-        unpack8(__ldg(raw_global + static_cast<int64_t>(r) * vectors_per_row + v), raw_bf16, f);
+        unpack8(load_global_v4(raw_global + static_cast<int64_t>(r) * vectors_per_row + v), raw_bf16, f);
         const auto exact = [=](float value) { return quantize_token_value(value, scale, inv_scale); };
         const uint32_t lo = quantize4(f[0], f[1], f[2], f[3], inv_scale, exact);
         const uint32_t hi = quantize4(f[4], f[5], f[6], f[7], inv_scale, exact);

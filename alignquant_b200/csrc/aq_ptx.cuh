@@ -101,5 +101,36 @@ __device__ __forceinline__ void grid_dependency_wait() {
 __device__ __forceinline__ void grid_launch_dependents() {
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
 }
+// Loads of what the preceding kernel writes.  Under dependent launch it may still be writing while this one is
+// resident: the read-only path (__ldg, or what the compiler makes of a const __restrict__ pointer) may return what
+// the line held before, and may be moved in front of grid_dependency_wait.  These do neither.
+__device__ __forceinline__ uint4 load_global_v4(const void* p) {
+  uint4 v;
+  asm volatile("ld.global.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+__device__ __forceinline__ uint2 load_global_v2(const void* p) {
+  uint2 v;
+  asm volatile("ld.global.v2.u32 {%0, %1}, [%2];" : "=r"(v.x), "=r"(v.y) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+__device__ __forceinline__ uint32_t load_global_u32(const void* p) {
+  uint32_t v;
+  asm volatile("ld.global.u32 %0, [%1];" : "=r"(v) : "l"(__cvta_generic_to_global(p)));
+  return v;
+}
+// Zeros where there is nothing to load.  By a predicate: with a branch around each load the loads of a lane are not
+// on their way together.
+__device__ __forceinline__ uint4 load_global_v4_if(const void* p, bool there) {
+  uint4 v;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "setp.ne.u32 p, %5, 0;\n\t"
+      "mov.u32 %0, 0;\n\tmov.u32 %1, 0;\n\tmov.u32 %2, 0;\n\tmov.u32 %3, 0;\n\t"
+      "@p ld.global.v4.u32 {%0, %1, %2, %3}, [%4];\n\t}"
+      : "=&r"(v.x), "=&r"(v.y), "=&r"(v.z), "=&r"(v.w)
+      : "l"(__cvta_generic_to_global(p)), "r"(static_cast<uint32_t>(there)));
+  return v;
+}
 
 }  // namespace aq

@@ -22,8 +22,8 @@ __device__ __forceinline__ void load16(const T* p, float (&v)[16]);
 
 template <>
 __device__ __forceinline__ void load16<__half>(const __half* p, float (&v)[16]) {
-  const uint4 a = __ldg(reinterpret_cast<const uint4*>(p));
-  const uint4 b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+  const uint4 a = load_global_v4(p);
+  const uint4 b = load_global_v4(p + 8);
   const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -36,8 +36,8 @@ __device__ __forceinline__ void load16<__half>(const __half* p, float (&v)[16]) 
 
 template <>
 __device__ __forceinline__ void load16<__nv_bfloat16>(const __nv_bfloat16* p, float (&v)[16]) {
-  const uint4 a = __ldg(reinterpret_cast<const uint4*>(p));
-  const uint4 b = __ldg(reinterpret_cast<const uint4*>(p) + 1);
+  const uint4 a = load_global_v4(p);
+  const uint4 b = load_global_v4(p + 8);
   const uint32_t w[8] = {a.x, a.y, a.z, a.w, b.x, b.y, b.z, b.w};
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -50,11 +50,11 @@ template <>
 __device__ __forceinline__ void load16<float>(const float* p, float (&v)[16]) {
 #pragma unroll
   for (int i = 0; i < 4; ++i) {
-    const float4 f = __ldg(reinterpret_cast<const float4*>(p) + i);
-    v[4 * i] = f.x;
-    v[4 * i + 1] = f.y;
-    v[4 * i + 2] = f.z;
-    v[4 * i + 3] = f.w;
+    const uint4 f = load_global_v4(p + 4 * i);
+    v[4 * i] = __uint_as_float(f.x);
+    v[4 * i + 1] = __uint_as_float(f.y);
+    v[4 * i + 2] = __uint_as_float(f.z);
+    v[4 * i + 3] = __uint_as_float(f.w);
   }
 }
 
@@ -178,7 +178,7 @@ __global__ void __launch_bounds__(256) quantize_token_rows_kernel(const T* __res
   const uint4* xr = reinterpret_cast<const uint4*>(x + row * k);
   uint4 raw[VECS];
 #pragma unroll
-  for (int i = 0; i < VECS; ++i) raw[i] = lane + kLanes * i < vectors ? __ldg(xr + lane + kLanes * i) : make_uint4(0, 0, 0, 0);
+  for (int i = 0; i < VECS; ++i) raw[i] = load_global_v4_if(xr + lane + kLanes * i, lane + kLanes * i < vectors);
   Pair most = *reinterpret_cast<const Pair*>(&raw[0].x);
   most = __habs2(most);
 #pragma unroll
@@ -397,7 +397,7 @@ __global__ void __launch_bounds__(256) rmsnorm_quantize_rows_kernel(const T* __r
   const uint4* wr = reinterpret_cast<const uint4*>(weight);
   uint4 raw[VECS];
 #pragma unroll
-  for (int i = 0; i < VECS; ++i) raw[i] = lane + kLanes * i < vectors ? __ldg(xr + lane + kLanes * i) : make_uint4(0, 0, 0, 0);
+  for (int i = 0; i < VECS; ++i) raw[i] = load_global_v4_if(xr + lane + kLanes * i, lane + kLanes * i < vectors);
   double even = 0.0, odd = 0.0;
 #pragma unroll
   for (int i = 0; i < VECS; ++i) {
@@ -491,13 +491,17 @@ __device__ __forceinline__ int quantize_fp64(double v, double scale, double inv_
 __device__ __noinline__ int quantize_fp64_call(double v, double scale, double inv_scale) { return quantize_fp64(v, scale, inv_scale); }
 
 __device__ __forceinline__ float2 load_pair(const __half* p) {
-  return __half22float2(__ldg(reinterpret_cast<const __half2*>(p)));
+  const uint32_t w = load_global_u32(p);
+  return __half22float2(*reinterpret_cast<const __half2*>(&w));
 }
 __device__ __forceinline__ float2 load_pair(const __nv_bfloat16* p) {
-  const uint32_t w = __ldg(reinterpret_cast<const uint32_t*>(p));
+  const uint32_t w = load_global_u32(p);
   return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u));
 }
-__device__ __forceinline__ float2 load_pair(const float* p) { return __ldg(reinterpret_cast<const float2*>(p)); }
+__device__ __forceinline__ float2 load_pair(const float* p) {
+  const uint2 w = load_global_v2(p);
+  return make_float2(__uint_as_float(w.x), __uint_as_float(w.y));
+}
 
 constexpr int kTileWarps = 4;  // warps (= tiles) of a CTA
 // A staged row: elements 32 .. 63 begin 16 floats late and rows are 81 floats apart, so that lanes
@@ -677,7 +681,8 @@ __global__ void __launch_bounds__(32 * kTileWarps) quantize_tile_kernel(const T*
 // numbers: as few lanes per row as leave each one to three vectors, so that no lane is idle (us at 16384 x
 // 512 with 1 / 2 / 4 / 8 warps per row: 8.0 / 10.6 / 16.3 / 26.7; 2048 x 3072: 11.5 / 8.2 / 6.5 / 7.5; 8192 x
 // 8192: - / 51.3 / 36.7 / 35.2).  Up to 1024 rows the longest row chain counts, not the lanes: a CTA
-// per row (75 x 2560: 4.5 / 3.0 / 2.3 / 1.9).
+// per row (75 x 2560: 4.5 / 3.0 / 2.3 / 1.9).  Vectors that a row does not have cost registers, and with them rows on
+// their way (2048 x 17408 with 16 / 12 vectors: 28.6 / 23.0).
 constexpr int64_t kRowKernelMaxK = 32768;
 
 template <typename Kernel>
@@ -692,6 +697,7 @@ struct RowLaunch {
    : (k) <= 2048               ? RowLaunch<decltype(&KERNEL<T, 1, 2>)>{KERNEL<T, 8, 1>, 8} \
    : (k) <= 8192               ? RowLaunch<decltype(&KERNEL<T, 1, 2>)>{KERNEL<T, 8, 4>, 8} \
    : (k) <= 16384              ? RowLaunch<decltype(&KERNEL<T, 1, 2>)>{KERNEL<T, 8, 8>, 8} \
+   : (k) <= 24576              ? RowLaunch<decltype(&KERNEL<T, 1, 2>)>{KERNEL<T, 8, 12>, 8} \
                                : RowLaunch<decltype(&KERNEL<T, 1, 2>)>{KERNEL<T, 8, 16>, 8})
 
 template <typename T>
