@@ -122,6 +122,9 @@ __global__ void __launch_bounds__(256) repack_kernel(
       dst[threadIdx.x] = make_uint4(out[0], out[1], out[2], out[3]);
     }
   }
+  // The projections fetch the image before their grid_dependency_wait, so the wait is not what makes it visible to
+  // them: it has to have reached device scope when the last CTA ends, which is when a dependent kernel may begin.
+  __threadfence();
 }
 
 }  // namespace

@@ -164,6 +164,11 @@ AQ_API int64_t aq_prepared_bytes(int32_t n_j, int32_t n_k, int64_t t4, int64_t t
  * chunk c = k/16 of row n stored at slot c ^ ((n/2) % 4).  W4 tile = 2048 B: 64 rows of
  * 32 bytes, byte 16h+i of row n = (w[n][32h+i] & 15) | (w[n][32h+16+i] << 4).
  * `prepared` must be 256-byte aligned and at least aq_prepared_bytes() long.
+ *
+ * The projections are launched as dependents of the kernel before them in the stream and fetch the
+ * image while that kernel still runs.  Behind aq_repack, a copy, or other work that has completed,
+ * that needs nothing; where a kernel of the caller's own writes or changes an image, synchronise
+ * with it (or put a copy or memset behind it) before the next projection is enqueued.
  */
 AQ_API int aq_repack(const uint8_t* state_bits, const uint8_t* w4_payload, const float* w4_scales,
               const int8_t* w8_payload, const float* w8_scales,

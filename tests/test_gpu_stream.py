@@ -7,6 +7,7 @@ import numpy as np
 import pytest
 import torch
 
+from alignquant_b200 import _lib
 from alignquant_b200.synthetic import synthetic_module_tensors
 from oracle import alignquant_oracle as oc
 from tests import helpers
@@ -515,3 +516,33 @@ def test_chained_calls_read_what_the_call_before_has_just_written(ext, scale_mod
         torch.cuda.synchronize()
         assert torch.equal(x, want)
     ext.device_status()
+
+
+@pytest.mark.parametrize("m", [1, 16, 32, 48, 128, 300])
+def test_image_can_be_laid_out_again_right_in_front_of_a_projection(ext, m):
+    """aq_repack of two layers in turn into one image, each followed at once by a projection, which fetches the
+    image ahead of its dependency: twenty times the result of an image of each layer's own."""
+    lib = _lib.load()
+    n, k = 1280, 512
+    n_j, n_k = n // 64, k // 64
+    x = torch.randn(m, k, generator=torch.Generator(device="cuda").manual_seed(m), device="cuda").half()
+    q, s = ext.alignquant_activation_quantize_cuda(x, None, scale_mode="token")
+    layers = []
+    for seed in (3, 4):
+        packed, _, _, _ = oc.synthetic_layer(n, k, seed=seed, w4_fraction=0.5)
+        weights, tensors = helpers.prepare_layer(packed, n_k)
+        layers.append((weights, tensors, ext.alignquant_linear_prepared(q, s, weights, None, scale_mode="token")))
+    weights = layers[0][0]
+    torch.cuda.synchronize()
+    haves = []
+    for _ in range(20):
+        for _, t, _ in layers:
+            status = lib.aq_repack(*(t[name].data_ptr() for name in ("state_bits", "w4_payload", "w4_scales", "w8_payload", "w8_scales",
+                                                                    "w4_row_offsets", "w8_row_offsets")), n_j, n_k,
+                                   t["w4_scales"].numel(), t["w8_scales"].numel(), weights.image.data_ptr(), weights.image.numel(),
+                                   torch.cuda.current_stream().cuda_stream)
+            assert status == 0, _lib.last_error()
+            haves.append(ext.alignquant_linear_prepared(q, s, weights, None, scale_mode="token"))
+    torch.cuda.synchronize()
+    ext.device_status()
+    assert all(torch.equal(have, layers[i % 2][2]) for i, have in enumerate(haves))
