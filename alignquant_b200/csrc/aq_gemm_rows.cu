@@ -122,7 +122,6 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap x_map, const RowsParams p) 
   auto acc_empty = [&](int b) { return bar0 + 8u * (3 * kStages + 2 + b); };
   const uint32_t final_bar = bar0 + 8u * (3 * kStages + 4);
 
-  grid_launch_dependents();
   if (threadIdx.x < S::kNumBars) {
     const int i = threadIdx.x;
     const bool of_widen = i >= kStages && i < 2 * kStages;
@@ -142,6 +141,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap x_map, const RowsParams p) 
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // Not before the allocation: a dependent kernel that shares the SM and takes tensor memory itself would get it first
+  // and keep it while it waits for this grid.
+  grid_launch_dependents();
   bool ok = true;
 
   if (warp >= kDrainWarps) {

@@ -309,7 +309,6 @@ tmem_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
   auto acc_empty = [&](int b) { return bar0 + 8u * (2 * kStages + kAccs + b); };
   const uint32_t final_bar = bar0 + 8u * (2 * kStages + 2 * kAccs);
 
-  grid_launch_dependents();
   // one thread per barrier: the initialisations would otherwise run one after the other
   if (threadIdx.x < S::kNumBars) {
     const int i = threadIdx.x;
@@ -331,6 +330,9 @@ tmem_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem_base = *tmem_slot;
+  // Not before the allocation: a dependent kernel that shares the SM and takes tensor memory itself would get it first
+  // and keep it while it waits for this grid.
+  grid_launch_dependents();
   bool ok = true;
 
   if (warp >= kDrainWarps) {
