@@ -723,8 +723,9 @@ constexpr int64_t kScratchBytes = 64LL << 20;
 // Tile rows per pass, the passes of about one size: the tile width and the K ranges are chosen for a pass.
 int rows_per_pass(int n_j, int n_k) {
   if (n_k > kMaxNk) return n_j;  // refused at the launch; a scratch of this size holds at least 24 tile rows up to there
-  const int64_t most = kScratchBytes / (static_cast<int64_t>(n_k) * kW8TileBytes) / 12 * 12;  // whole CTA tiles of every width
+  int64_t most = kScratchBytes / (static_cast<int64_t>(n_k) * kW8TileBytes);
   if (most >= n_j) return n_j;
+  most = most / 12 * 12;  // whole CTA tiles of every width
   const int64_t passes = (n_j + most - 1) / most;
   return static_cast<int>(((n_j + passes - 1) / passes + 11) / 12 * 12);
 }
@@ -919,7 +920,10 @@ GemmPlan plan_gemm(int64_t m, int n_j, int n_k) {
       return plan;
     }
   }
-  plan.workspace_bytes = kScratchOffset + static_cast<int64_t>((plan.rows_per_pass + 11) / 12 * 12) * n_k * kW8TileBytes;
+  // Up to three tile rows fill up the last CTA tile.  A layer that is cut into passes asks for the whole scratch, not
+  // for its longest pass, so that what suffices for a layer suffices for every smaller one.
+  const int64_t tile_row = static_cast<int64_t>(n_k) * kW8TileBytes;
+  plan.workspace_bytes = kScratchOffset + (plan.rows_per_pass == n_j ? n_j * tile_row : kScratchBytes) + 3 * tile_row;
   return plan;
 }
 

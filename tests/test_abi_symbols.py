@@ -36,6 +36,21 @@ def test_pure_host_entry_points():
     assert lib.aq_linear_workspace_bytes(64, 4, 4, 0, 4) == 0  # explicit splits: cluster kernel, no scratch
 
 
+@pytest.mark.parametrize("m", [33, 129, 4096])
+def test_workspace_of_the_largest_layer_suffices_for_smaller_ones(m):
+    """One buffer serves every layer: the size does not fall as a layer gets wider or longer, whatever passes it is cut into."""
+    size = _lib.load().aq_linear_workspace_bytes
+    widths = [*range(1, 40), 79, 80, 204, 205, 408, 409, 420, 544, 819, 1024, 2500]
+    lengths = [1, 2, 3, 31, 40, 79, 80, 81, 127, 160, 272, 333, 334, 335, 340, 342, 455, 456, 500, 511, 512]
+    table = [[size(m, n_j, n_k, 0, 0) for n_k in lengths] for n_j in widths]
+    if m > 128:  # at fewer rows some layers take the kernel without a workspace
+        assert all(a <= b for row in table for a, b in zip(row, row[1:]))
+        assert all(a <= b for upper, lower in zip(table, table[1:]) for a, b in zip(upper, lower))
+    most = size(4096, 2500, 512, 0, 0)
+    assert 0 <= min(map(min, table)) and max(map(max, table)) <= most
+    assert f"{most // 1000000} {most // 1000 % 1000:03d} {most % 1000:03d} bytes" in HEADER.read_text()
+
+
 @pytest.mark.parametrize("n_k", [513, 1365, 1366, 20000])
 @pytest.mark.parametrize("m,schedule", [(33, 0), (128, 0), (129, 0), (4096, 0), (2, 3), (129, 3)])
 def test_k_above_the_gemm_limit_is_refused_with_a_message(m, schedule, n_k):
