@@ -376,7 +376,9 @@ __global__ void __launch_bounds__(256) rmsnorm_quantize_kernel(const T* __restri
 // The same for rows of up to 32768 16-bit values, with the layout of quantize_token_rows_kernel.  The normalised
 // row, already rounded to T, takes the place of the loaded one in the lane's registers.  Bound by the
 // conversions to FP64 (a quarter or less of the full rate; their unit is busy half of the time): 16384 x 2560 bf16
-// 147 -> 62 us, 8192 x 8192 136 -> 75.
+// 147 -> 62 us, 8192 x 8192 136 -> 75.  So a lane's empty places count: they are as few as the layouts allow, and skipped
+// where there may be many (2048 x 17408: 85 us with a CTA that reads its row twice, 93 with 16 vectors per lane,
+// 81 with twelve, 44 with the empty ones skipped; 1024 x 2560 with four / two vectors 7.8 / 5.8).
 template <typename T, int WARPS, int VECS>
 __global__ void __launch_bounds__(256) rmsnorm_quantize_rows_kernel(const T* __restrict__ x, const T* __restrict__ weight,
                                                                     float eps, int8_t* __restrict__ q,
@@ -401,6 +403,7 @@ __global__ void __launch_bounds__(256) rmsnorm_quantize_rows_kernel(const T* __r
   double even = 0.0, odd = 0.0;
 #pragma unroll
   for (int i = 0; i < VECS; ++i) {
+    if (VECS > 8 && kLanes * i >= vectors) break;  // no FP64 for what the row does not have
     float v[8];
     unpack8(raw[i], kBf16, v);
 #pragma unroll
@@ -695,6 +698,7 @@ struct RowLaunch {
    : (m) > 1024 && (k) <= 1024 ? RowLaunch<decltype(&KERNEL<T, 1, 2>)>{KERNEL<T, 2, 2>, 2} \
    : (m) > 1024 && (k) <= 4096 ? RowLaunch<decltype(&KERNEL<T, 1, 2>)>{KERNEL<T, 4, 4>, 4} \
    : (k) <= 2048               ? RowLaunch<decltype(&KERNEL<T, 1, 2>)>{KERNEL<T, 8, 1>, 8} \
+   : (k) <= 4096               ? RowLaunch<decltype(&KERNEL<T, 1, 2>)>{KERNEL<T, 8, 2>, 8} \
    : (k) <= 8192               ? RowLaunch<decltype(&KERNEL<T, 1, 2>)>{KERNEL<T, 8, 4>, 8} \
    : (k) <= 16384              ? RowLaunch<decltype(&KERNEL<T, 1, 2>)>{KERNEL<T, 8, 8>, 8} \
    : (k) <= 24576              ? RowLaunch<decltype(&KERNEL<T, 1, 2>)>{KERNEL<T, 8, 12>, 8} \

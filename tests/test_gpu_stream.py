@@ -146,7 +146,7 @@ def _run_linear(ext, xq, a_s, weights, u_meta, m, n_j, n_k, **kw):
 
 
 @pytest.mark.parametrize("dtype", [torch.bfloat16, torch.float16])
-@pytest.mark.parametrize("m,k", [(1024, 512), (1025, 64), (1031, 512), (1025, 576), (1025, 1024), (1027, 1088), (1026, 4096),
+@pytest.mark.parametrize("m,k", [(1024, 512), (1025, 64), (1031, 512), (1025, 576), (1025, 1024), (1027, 1088), (1026, 4096), (1024, 4096), (1024, 4160), (3, 17408),
                                  (1025, 4160), (3, 2048), (3, 2112), (5, 8192), (3, 8256), (2, 16384), (2, 16448), (2, 24576), (2, 24640), (2, 32768), (2, 32832)])
 def test_row_quantizers_at_the_borders_of_their_layouts(ext, m, k, dtype):
     """Every number of warps per row and of vectors per lane, with the last lanes full and nearly empty, and
