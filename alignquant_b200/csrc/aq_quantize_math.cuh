@@ -30,14 +30,15 @@ __device__ __forceinline__ uint32_t pack4(int a, int b, int c, int d) {
 
 // Four values -> four int8 codes.  v * inv is rounded to a whole number by adding 1.5 * 2^23 (one
 // fused multiply-add; the code is the low byte of the sum), the distance to it by a second one.  The
-// callers' inv differs from 1 / scale by less than 2^-22 of it and |v / scale| < 129, so the distance
-// is off by less than 4e-5: below 0.5 - 1e-4 the code is that of the exact quotient and lies in
-// the code's range.  Otherwise (and for NaN) all four go to `exact`.  Full-rate instructions only:
+// callers' inv is 1 / scale to 2^-24 of it (one rounding) and |v / scale| <= 128, so v * inv is off by 2^-17, the
+// distance by 2^-26 more and, where `exact` rounds the quotient to FP32 first, that by 2^-18: below 0.5 - 2^-16 the
+// code is that of `exact` and lies in its range.  Otherwise (and for NaN) all four go to `exact`.  Every value
+// that goes there counts in a launch of two microseconds (with 1e-4 in place of 2^-16: 32 x 5120 bf16 2.5, now 1.9).  Full-rate instructions only:
 // conversions to and from integers run at a quarter of the rate and, with the compares, clamps and
 // masks of quantize_token_value, bounded the quantizers (8192 x 8192 bf16: 59 us).
 template <typename Exact>
 __device__ __forceinline__ uint32_t quantize4(float v0, float v1, float v2, float v3, float inv, Exact exact) {
-  constexpr float kMagic = 12582912.0f, kClear = 0.5f - 1.0e-4f;
+  constexpr float kMagic = 12582912.0f, kClear = 0.5f - 1.0f / 65536.0f;
   const float m0 = __fmaf_rn(v0, inv, kMagic), m1 = __fmaf_rn(v1, inv, kMagic);
   const float m2 = __fmaf_rn(v2, inv, kMagic), m3 = __fmaf_rn(v3, inv, kMagic);
   const float d0 = __fmaf_rn(v0, inv, __fsub_rn(kMagic, m0)), d1 = __fmaf_rn(v1, inv, __fsub_rn(kMagic, m1));

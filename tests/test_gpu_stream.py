@@ -125,6 +125,28 @@ def test_tile_quantizer_bit_exact_identity(ext, m, k, dtype):
     assert np.array_equal(q.cpu().numpy(), q_ref[:m])
 
 
+@pytest.mark.parametrize("dtype", [torch.float16, torch.bfloat16, torch.float32])
+@pytest.mark.parametrize("side", [127.0, -128.0])
+def test_tile_quantizer_rounding_boundaries(ext, dtype, side):
+    """Quotients on and next to .5 boundaries of every code, for maxima with few and with many bits, on either side of
+    zero: the codes of an FP64 division rounded to even."""
+    m, k = 16 * 24, 320
+    rng = np.random.default_rng(5)
+    extreme = np.sign(side) * np.exp2(rng.integers(-4, 5, (24, 1, k // 64, 1))) * rng.choice([1.0, 1.5, 1.25, 1.0078125, 1.984375], (24, 1, k // 64, 1))
+    targets = rng.integers(-127, 127, (24, 16, k // 64, 64)) + 0.5
+    x = torch.from_numpy(targets * (extreme / side)).to(dtype)
+    steps = torch.from_numpy(rng.integers(-1, 2, x.shape).astype(np.int32 if dtype == torch.float32 else np.int16))
+    x = (x.view(steps.dtype) + steps).view(dtype)  # the neighbours of the dtype
+    bound = torch.from_numpy(np.abs(extreme)).to(dtype)
+    x = torch.clamp(x, -bound, bound)
+    x[:, :1, :, :1] = torch.from_numpy(extreme).to(dtype)
+    x = x.reshape(m, k).contiguous()
+    q, s = ext.alignquant_activation_quantize_cuda(x.cuda(), None)
+    q_ref, s_ref = oc.a8_tile_quantize(x.double().numpy())
+    assert np.array_equal(s.cpu().numpy().reshape(s_ref.shape), s_ref)
+    assert np.array_equal(q.cpu().numpy(), q_ref)
+
+
 def test_tile_quantizer_matches_reference_fixture_with_transform(ext, golden_dir):
     g = dict(np.load(golden_dir / "act_quant_mixed.npz"))
     xt = torch.from_numpy(g["x"]).cuda()
