@@ -3,7 +3,10 @@
 // With few rows the weights are the large operand: they are read once, straight from the prepared
 // image, and they are the M side of the MMA.  A CTA takes two tile rows (128 output columns) and a
 // range of K; D is 128 columns x NT activation rows (NT = 32, 64 or 128), so nothing is spent on
-// padding the rows to 128.  What bounds it is the weight stream; the GEMM of aq_gemm_tmem.cu expands the
+// padding the rows to 128.  Above 64 rows there is no padding to save and the sides change: with the rows on the M side
+// a drain lane has one row and one tile row, so that one scale serves all of its results of a step (with the
+// weights there, a multiplication and a shared-memory read for every pair of results: 1060 cycles a step, now 660).  What
+// bounds it is the weight stream; the GEMM of aq_gemm_tmem.cu expands the
 // weights into a workspace first (2.4 times the bytes written and read again) and drains 128 x 256 results
 // per step whatever the rows: 34816 x 5120 at 48 rows took 167 us there.
 //
@@ -13,9 +16,9 @@
 //     the eight meet at a barrier, then each lays its tile down in its operand slot (64-byte swizzle, W4 as 16*w);
 //   * one warp issues tcgen05.mma kind::i8 (M = 128, N = NT, K = 32) into one of two accumulators of
 //     SUB x NT columns: a hand-over covers a whole stage;
-//   * eight warps drain: 32 columns x NT / 2 rows each, one packed multiply (activation scale x
-//     weight scale) and one packed fused multiply-add per two results, tiles in increasing k: the
-//     roundings of aq_gemm_tmem.cu, bit for bit;
+//   * eight warps drain: 32 columns x NT / 2 rows each (NT = 128: 32 rows x 64 columns), one packed multiply
+//     (activation scale x weight scale; NT = 128: one per step) and one packed fused multiply-add per two results,
+//     tiles in increasing k: the roundings of aq_gemm_tmem.cu, bit for bit;
 //   * K ranges of a thread-block cluster meet in distributed shared memory, added in split order.
 //
 // Every wait is bounded, as in aq_gemm_tmem.cu.
@@ -50,7 +53,6 @@ constexpr int kOtherRegs = 64;
 static_assert(kDrainWarps * 32 * kDrainRegs + (kThreads - kDrainWarps * 32) * kOtherRegs <= kThreads * 96,
               "setmaxnreg would wait for registers that the block does not have");
 constexpr int kMmaRows = 2 * kTile;  // output columns of a CTA: the M side of the MMA
-constexpr int kXchgRow = kMmaRows + 4;  // floats per activation row of the exchange tile
 
 template <int NT>
 struct RowsLayout {
@@ -62,7 +64,9 @@ struct RowsLayout {
   static constexpr int kAccColumns = kSub * NT;              // at most 256
   static constexpr int kTmemColumns = 2 * kAccColumns;
   static constexpr int kWarpsPerTile = kWidenWarps / (2 * kSub);
-  static constexpr int kCols = NT / 2;                       // activation rows of a drain warp
+  static constexpr bool kRowsOnM = NT == 128;                // lanes of an accumulator: activation rows, else output columns
+  static constexpr int kCols = NT / 2;                       // accumulator columns of a drain warp (activation rows; kRowsOnM: output columns)
+  static constexpr int kXchgRow = kMmaRows + (kRowsOnM ? 1 : 4);  // floats per activation row of the exchange tile
   // landed[S], ready[S], empty[S], acc_full[2], acc_empty[2], final
   static constexpr int kNumBars = 3 * kStages + 5;
   static constexpr int kSmemBytes = kStages * kStageBytes + NT * 4 + kNumBars * 8 + 16;
@@ -224,8 +228,8 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap x_map, const RowsParams p) 
             const uint64_t a_desc = a_desc0 + (stage + s * (2 * kW8TileBytes / 16));
             const uint64_t b_desc = b_desc0 + (stage + s * (NT * kTile / 16));
             const uint32_t d = tmem_base + b * S::kAccColumns + static_cast<uint32_t>(s * NT);
-            tc_mma_i8(d, a_desc, b_desc, idesc, 0u);
-            tc_mma_i8(d, a_desc + 2, b_desc + 2, idesc, 1u);
+            tc_mma_i8(d, S::kRowsOnM ? b_desc : a_desc, S::kRowsOnM ? a_desc : b_desc, idesc, 0u);
+            tc_mma_i8(d, (S::kRowsOnM ? b_desc : a_desc) + 2, (S::kRowsOnM ? a_desc : b_desc) + 2, idesc, 1u);
           }
         }
         tc_commit(acc_full(b));
@@ -304,18 +308,22 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap x_map, const RowsParams p) 
   }
   } else {
     asm volatile("setmaxnreg.inc.sync.aligned.u32 %0;" ::"n"(kDrainRegs));
-    // ---------------- drain: lane = output column, registers = activation rows -------------------
+    // ---------------- drain: lane = output column, registers = activation rows; kRowsOnM: the other way round ----------
     constexpr int kCols = S::kCols;
+    constexpr bool kRowsOnM = S::kRowsOnM;
+    constexpr int kXchgRow = S::kXchgRow;
     const int quarter = warp & 3;  // tensor-memory lane quarter this warp may read
-    const int group = warp >> 2;   // activation rows group * kCols ..
-    const int j = j0 + (quarter >> 1);
+    const int group = warp >> 2;   // accumulator columns group * kCols ..
+    const int j = j0 + (kRowsOnM ? group : quarter >> 1);
     const TileRecord* recs = p.records + static_cast<int64_t>(j < p.n_j ? j : j0) * n_k + k_begin;
     const uint32_t taddr = tmem_base + (static_cast<uint32_t>(quarter * 32) << 16) + static_cast<uint32_t>(group * kCols);
     float w_next[kSub];
 #pragma unroll
     for (int s = 0; s < kSub; ++s) w_next[s] = s < steps ? __ldg(&recs[s].scale) : 0.0f;
     grid_dependency_wait();  // the activation scales come from the preceding kernel, and it may read what is stored here
-    constexpr int kRowGroups = kCols / 16;  // 16-row groups of the warp, one scale each per step under tile scales
+    // 16-row groups of the warp (kRowsOnM: of the lane), one scale each per step under tile scales
+    constexpr int kRowGroups = kRowsOnM ? 1 : kCols / 16;
+    const int m_row = quarter * 32 + lane;  // kRowsOnM: this lane's activation row
     float g_next[kToken ? 1 : kSub][kRowGroups];
     // Ordinary loads, as for all that the preceding kernel writes: it may still be writing while this one is resident,
     // and the read-only path does not see that (stale scales at 128 x 3072 x 3072).
@@ -325,7 +333,7 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap x_map, const RowsParams p) 
         for (int s = 0; s < kSub; ++s) {
 #pragma unroll
           for (int g = 0; g < kRowGroups; ++g) {
-            const int row_group = group * kRowGroups + g;
+            const int row_group = kRowsOnM ? m_row >> 4 : group * kRowGroups + g;
             g_next[s][g] = at + s < steps && row_group * 16 < p.m
                                ? p.act_scales[static_cast<int64_t>(row_group) * n_k + k_begin + at + s]
                                : 0.0f;
@@ -334,7 +342,10 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap x_map, const RowsParams p) 
       }
     };
     group_scales(0);
-    if (kToken) {
+    float token_scale = 0.0f;
+    if constexpr (kToken && kRowsOnM) {
+      if (m_row < p.m) token_scale = p.act_scales[m_row];
+    } else if (kToken) {
       if (threadIdx.x < NT) row_scales[threadIdx.x] = static_cast<int>(threadIdx.x) < p.m ? p.act_scales[threadIdx.x] : 0.0f;
       asm volatile("bar.sync 2, %0;" ::"n"(kDrainWarps * 32) : "memory");
     }
@@ -386,11 +397,13 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap x_map, const RowsParams p) 
           for (int h = 0; h < kSteps; ++h) {
             const int s = s0 + h;
             if (at + s >= steps) break;
-            const uint64_t w2 = both(w_s[s]);
+            const uint64_t w2 = kRowsOnM ? both(__fmul_rn(kToken ? token_scale : g_s[kToken ? 0 : s][0], w_s[s])) : both(w_s[s]);
 #pragma unroll
             for (int i = 0; i < kPart; i += 4) {
               uint64_t scale_a, scale_b;
-              if constexpr (kToken) {
+              if constexpr (kRowsOnM) {
+                scale_a = scale_b = w2;
+              } else if constexpr (kToken) {
                 const ulonglong2 a = my_scales[(c0 + i) / 4];
                 scale_a = mul2(a.x, w2);
                 scale_b = mul2(a.y, w2);
@@ -408,10 +421,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap x_map, const RowsParams p) 
               const int shift = (recs[at + s].offset_flag & kW4Flag) ? 4 : 0;
 #pragma unroll
               for (int i = 0; i < kPart; ++i) {
-                const int row = group * kCols + c0 + i;
-                if (row < p.m) {
-                  p.acc_dump[((static_cast<int64_t>(row) * p.n_j + j) * n_k + k) * kTile + (quarter & 1) * 32 + lane] = v[h][i] >> shift;
-                }
+                const int row = kRowsOnM ? m_row : group * kCols + c0 + i;
+                const int column = kRowsOnM ? c0 + i : (quarter & 1) * 32 + lane;
+                if (row < p.m) p.acc_dump[((static_cast<int64_t>(row) * p.n_j + j) * n_k + k) * kTile + column] = v[h][i] >> shift;
               }
             }
           }
@@ -428,8 +440,9 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap x_map, const RowsParams p) 
     for (int i = 0; i < kCols / 2; ++i) {
       float lo, hi;
       unpack2(acc[i], lo, hi);
-      xchg[(group * kCols + 2 * i) * kXchgRow + quarter * 32 + lane] = lo;
-      xchg[(group * kCols + 2 * i + 1) * kXchgRow + quarter * 32 + lane] = hi;
+      const int column = group * kCols + 2 * i;  // of the accumulator
+      xchg[kRowsOnM ? m_row * kXchgRow + column : column * kXchgRow + quarter * 32 + lane] = lo;
+      xchg[kRowsOnM ? m_row * kXchgRow + column + 1 : (column + 1) * kXchgRow + quarter * 32 + lane] = hi;
     }
   }
   if (*abort_flag != 0) {
@@ -454,33 +467,68 @@ gemm_rows_kernel(const __grid_constant__ CUtensorMap x_map, const RowsParams p) 
 #pragma unroll
     for (int s = 0; s < 8; ++s) remote[s] = split_k > 1 ? cluster.map_shared_rank(xchg, s < split_k ? s : 0) : xchg;
     const int64_t n_cols = static_cast<int64_t>(p.n_j) * kTile;
-    for (int q = warp; q < owned * tiles_here; q += kDrainWarps) {
-      const int row = split + split_k * (q / tiles_here);
-      const int tl = q % tiles_here;
-      const int offset = row * kXchgRow + tl * kTile + lane;
-      float a[8], b[8];
+    if (split_k == 1 && p.u_metadata == nullptr) {
+      // Eight warps do not hide chains of integer arithmetic: with the row, the tile row and the address worked out for
+      // every pair, as below, a pair takes 280 cycles, 9000 for a CTA of 128 rows (128 x 18944 x 1024 17.6 us, now 12.1).
+      constexpr int kTogether = 4;  // rows whose loads do not wait for the stores of the row before
+      const int tl = tiles_here == 2 ? warp & 1 : 0;
+      const int first = tiles_here == 2 ? warp >> 1 : warp, every = kDrainWarps / tiles_here;
+      const float* from = xchg + first * S::kXchgRow + tl * kTile + lane;
+      const int from_step = every * S::kXchgRow;
+      const int64_t to_step = every * n_cols;
+      auto store = [&](auto* out) {
+        int64_t to = first * n_cols + static_cast<int64_t>(j0 + tl) * kTile + lane;
+        int row = first;
+        for (; row + (kTogether - 1) * every < p.m; row += kTogether * every) {
+          float lo[kTogether], hi[kTogether];
 #pragma unroll
-      for (int s = 0; s < 8; ++s) {
-        a[s] = b[s] = 0.0f;
-        if (s < split_k) {
-          a[s] = remote[s][offset];
-          b[s] = remote[s][offset + 32];
-        }
-      }
-      float lo = a[0], hi = b[0];
+          for (int h = 0; h < kTogether; ++h, from += from_step) {
+            lo[h] = from[0];
+            hi[h] = from[32];
+          }
 #pragma unroll
-      for (int s = 1; s < 8; ++s) {
-        if (s < split_k) {
-          lo = __fadd_rn(lo, a[s]);
-          hi = __fadd_rn(hi, b[s]);
+          for (int h = 0; h < kTogether; ++h, to += to_step) {
+            store_out(out, to, lo[h]);
+            store_out(out, to + 32, hi[h]);
+          }
         }
+        for (; row < p.m; row += every, from += from_step, to += to_step) {
+          store_out(out, to, from[0]);
+          store_out(out, to + 32, from[32]);
+        }
+      };
+      if (p.out_dtype == AQ_F32) store(static_cast<float*>(p.out));
+      else if (p.out_dtype == AQ_BF16) store(static_cast<__nv_bfloat16*>(p.out));
+      else store(static_cast<__half*>(p.out));
+    } else {
+      for (int q = warp; q < owned * tiles_here; q += kDrainWarps) {
+        const int row = split + split_k * (q / tiles_here);
+        const int tl = q % tiles_here;
+        const int offset = row * S::kXchgRow + tl * kTile + lane;
+        float a[8], b[8];
+#pragma unroll
+        for (int s = 0; s < 8; ++s) {
+          a[s] = b[s] = 0.0f;
+          if (s < split_k) {
+            a[s] = remote[s][offset];
+            b[s] = remote[s][offset + 32];
+          }
+        }
+        float lo = a[0], hi = b[0];
+#pragma unroll
+        for (int s = 1; s < 8; ++s) {
+          if (s < split_k) {
+            lo = __fadd_rn(lo, a[s]);
+            hi = __fadd_rn(hi, b[s]);
+          }
+        }
+        const int j = j0 + tl;
+        const int32_t* meta = p.u_metadata ? p.u_metadata + static_cast<int64_t>(j) * 4 * kTile : nullptr;
+        if (meta != nullptr && meta[0] != 0) inverse_u_row(lo, hi, meta, lane);
+        const int64_t o = static_cast<int64_t>(row) * n_cols + static_cast<int64_t>(j) * kTile + lane;
+        store_any(p.out, p.out_dtype, o, lo);
+        store_any(p.out, p.out_dtype, o + 32, hi);
       }
-      const int j = j0 + tl;
-      const int32_t* meta = p.u_metadata ? p.u_metadata + static_cast<int64_t>(j) * 4 * kTile : nullptr;
-      if (meta != nullptr && meta[0] != 0) inverse_u_row(lo, hi, meta, lane);
-      const int64_t o = static_cast<int64_t>(row) * n_cols + static_cast<int64_t>(j) * kTile + lane;
-      store_any(p.out, p.out_dtype, o, lo);
-      store_any(p.out, p.out_dtype, o + 32, hi);
     }
   }
   if (split_k > 1) cluster.sync();
@@ -561,12 +609,13 @@ int resident_clusters(const Shape& shape, int split, int device) {
 
 }  // namespace
 
-// K ranges and their cost by a model in SM cycles: a K step of two tiles (measured 520, 650 and 1060 for 32, 64
-// and 128 rows), what a CTA costs beside its steps, the exchange; clusters in waves.
+// K ranges and their cost by a model in SM cycles: a K step of two tiles (measured 490, 560 and 660 for 32, 64
+// and 128 rows), what a CTA costs beside its steps, the exchange (more with every row that changes hands: 128 x 4736 x 5120
+// gains 9 us from a second range, which its steps alone would put at 14); clusters in waves.
 // `forced` (AQ_OPT_GEMM_SPLIT) >= 1: that number.
 int gemm_rows_split(int64_t m, int n_j, int n_k, int forced, double* cost) {
   const int pairs = (n_j + 1) / 2;
-  const double step = m <= 32 ? 520.0 : m <= 64 ? 650.0 : 1060.0;
+  const double step = m <= 32 ? 490.0 : m <= 64 ? 560.0 : 660.0;
   int device = 0;
   if (cudaGetDevice(&device) != cudaSuccess) device = 0;
   const Shape& shape = shape_for(m);
@@ -577,7 +626,7 @@ int gemm_rows_split(int64_t m, int n_j, int n_k, int forced, double* cost) {
     const int at_once = split == 1 ? num_sms() : resident_clusters(shape, split, device);
     if (at_once <= 0 && forced < 1) continue;
     const int waves = at_once > 0 ? (pairs + at_once - 1) / at_once : pairs;
-    const double this_cost = static_cast<double>(waves) * ((n_k + split - 1) / split * step + 7000.0) + (split > 1 ? 1500.0 : 0.0);
+    const double this_cost = static_cast<double>(waves) * ((n_k + split - 1) / split * step + 8000.0) + (split > 1 ? 1500.0 + 40.0 * static_cast<double>(m) : 0.0);
     if (best_cost == 0.0 || this_cost < best_cost) {
       best_cost = this_cost;
       best = split;

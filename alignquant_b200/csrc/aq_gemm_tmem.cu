@@ -892,9 +892,10 @@ Choice choose(int64_t m, int n_j, int n_k, int forced_tile, int forced_split, in
 }  // namespace
 
 // Up to 128 rows the kernel that reads the packed weights once, where that pass costs less than their expansion and
-// the GEMM for many rows, both by their models (expansion: 2.1 cycles per tile, measured: 14 us for 12288 tiles).
-// Measured (us, gemm_rows_kernel / the other): 48 rows 34816 x 5120 61 / 110, 5120 x 17408 34 / 82, 3072 x 3072 8.9 /
-// 12.9, 19456 x 2560 (152 CTAs: a second wave of four) 36 / 33; 75 rows 16384 x 3072 31 / 28.5.
+// the GEMM for many rows, both by their models (expansion: 2.1 cycles per tile, measured: 14 us for 12288 tiles, but not
+// less than 4000, and a launch).  Measured (us, gemm_rows_kernel / the other): 64 rows 34816 x 5120 57 / 91, 1024 x 1024
+// 6.1 / 9.4, 3072 x 3072 9.5 / 13; 128 rows 34816 x 5120 65 / 91, 16384 x 3072 21.5 / 28.4, 1024 x 1024 8.4 / 9.5,
+// 19456 x 64 8.9 / 7.2, 19456 x 2560 (152 CTAs: a second wave of four) 36 / 33.
 GemmPlan plan_gemm(int64_t m, int n_j, int n_k) {
   const int forced_tile = gemm_tile_option();
   const int forced_split = gemm_split_option();
@@ -911,7 +912,8 @@ GemmPlan plan_gemm(int64_t m, int n_j, int n_k) {
   if (n_k > kMaxNk) return plan;  // the launch says why
   if (m <= kBM && plan.fused && forced_tile == AQ_GEMM_TILE_AUTO) {
     const int passes = (n_j + plan.rows_per_pass - 1) / plan.rows_per_pass;
-    const double cost = passes * choice.cost + 2.1 * static_cast<double>(n_j) * n_k + 2000.0;
+    const double tiles = static_cast<double>(n_j) * n_k;
+    const double cost = passes * (choice.cost + 4500.0) + (2.1 * tiles > 4000.0 ? 2.1 * tiles : 4000.0);
     double rows_cost = 0.0;
     const int rows_split = gemm_rows_split(m, n_j, n_k, forced_split, &rows_cost);
     if (forced_split >= 1 || rows_cost < cost) {
