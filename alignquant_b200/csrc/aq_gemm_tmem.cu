@@ -716,9 +716,10 @@ __global__ void __launch_bounds__(256) expand_kernel(const TileRecord* __restric
 
 // The workspace starts with the arrival counters of the stream-K kernel, which have to stay zero.
 constexpr int64_t kScratchOffset = 64 * 1024;
-// Expanded weights at a time: a layer above this is run in several passes over its columns, each of
-// which finds its operand in the L2.
-constexpr int64_t kScratchBytes = 64LL << 20;
+// Expanded weights at a time: a layer above this is run in several passes over its columns.  Not so few that a pass
+// leaves SMs idle: with 64 MiB, which the L2 would keep, 129 x 34816 x 5120 ran three passes of 96 output tiles, 157
+// us against 127 in one, and 129 x 65536 x 2048 131 against 104.
+constexpr int64_t kScratchBytes = 256LL << 20;
 
 // Tile rows per pass, the passes of about one size: the tile width and the K ranges are chosen for a pass.
 int rows_per_pass(int n_j, int n_k) {
@@ -913,7 +914,9 @@ GemmPlan plan_gemm(int64_t m, int n_j, int n_k) {
   if (m <= kBM && plan.fused && forced_tile == AQ_GEMM_TILE_AUTO) {
     const int passes = (n_j + plan.rows_per_pass - 1) / plan.rows_per_pass;
     const double tiles = static_cast<double>(n_j) * n_k;
-    const double cost = passes * (choice.cost + 4500.0) + (2.1 * tiles > 4000.0 ? 2.1 * tiles : 4000.0);
+    // Above what the L2 keeps the expanded weights come from HBM again: 14000 cycles more, whatever the size.
+    const double again = static_cast<double>(plan.rows_per_pass) * n_k * kW8TileBytes > 64e6 ? 14000.0 : 0.0;
+    const double cost = passes * (choice.cost + again + 4500.0) + (2.1 * tiles > 4000.0 ? 2.1 * tiles : 4000.0);
     double rows_cost = 0.0;
     const int rows_split = gemm_rows_split(m, n_j, n_k, forced_split, &rows_cost);
     if (forced_split >= 1 || rows_cost < cost) {

@@ -501,7 +501,7 @@ def _takes_gemm(m: int, schedule_code: int) -> bool:
 def _workspace(device: torch.device, size: int, gemm: bool) -> torch.Tensor:
     """Scratch of one call.
 
-    The GEMM's (``gemm``: expanded weights, up to 64 MiB) needs no content: it is the caching
+    The GEMM's (``gemm``: expanded weights, up to 262 MiB) needs no content: it is the caching
     allocator's, taken and given back by every call like any temporary, so that streams, threads and captured graphs
     never meet in it.  The stream-K kernel's holds arrival counters that a call finds and leaves
     zeroed: one zeroed buffer per (device, stream), where calls run in order, which only grows.

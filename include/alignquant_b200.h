@@ -179,8 +179,8 @@ AQ_API int aq_repack(const uint8_t* state_bits, const uint8_t* w4_payload, const
 /*
  * Bytes of workspace aq_linear needs for this problem (0 when none is needed).  The
  * workspace holds per-row arrival counters (its first 64 KiB) followed by split-K
- * partial tiles or, for the GEMM, weights expanded to int8 (64 MiB and three rows of tiles, with the
- * counters at most 73 465 856 bytes: larger layers are run in several passes over their columns).  Its
+ * partial tiles or, for the GEMM, weights expanded to int8 (256 MiB and three rows of tiles, with the
+ * counters at most 274 792 448 bytes: larger layers are run in several passes over their columns).  Its
  * owner must zero it once before the first call; every call returns the counters to zero, so one
  * buffer can be reused by later calls on the same stream.  Above 32 rows the size does not fall as m,
  * n_j or n_k grow: what it is for the longest prompt and the largest layer suffices for all others.  It
