@@ -276,7 +276,45 @@ __device__ __forceinline__ void dump16(const GemmParams& p, int64_t row, int j, 
   }
 }
 
-template <int TN, bool kDump, bool kFused>
+// Output transforms of a finished 128-column tile whose FP32 sums lie in shared memory (rows of `stride` floats), where a
+// CTA has one output tile only and so the stage ring to put them in.  A warp takes 16 rows of one tile row; a pair
+// of lanes owns a row (lane 2 r + h its elements 32 h .. 32 h + 31), so that five of the six butterfly stages stay in
+// registers, in the order of inverse_u_row and with its roundings.  (inverse_u_row has two elements per lane and some
+// twenty dependent shuffles a row, 20 us for the 32 rows of a drain warp: 128 x 1024 x 1024 29.9 us, now 13.)
+__device__ __forceinline__ void turn_rows(float* sums, int stride, const int32_t* meta, int lane) {
+  const int half = lane & 1;
+  float* own = sums + (lane >> 1) * stride;
+  if (meta == nullptr || meta[0] == 0) return;
+  double e[32];
+#pragma unroll
+  for (int i = 0; i < 32; ++i) e[i] = static_cast<double>(own[32 * half + i]) * static_cast<double>(meta[3 * kTile + 32 * half + i]);
+#pragma unroll
+  for (int stride_of = 1; stride_of < 32; stride_of <<= 1) {
+#pragma unroll
+    for (int i = 0; i < 32; ++i) {
+      if ((i & stride_of) == 0) {
+        const double a = e[i], b = e[i + stride_of];
+        e[i] = a + b;
+        e[i + stride_of] = a - b;
+      }
+    }
+  }
+  __syncwarp();
+  // lane h ends up with elements 16 h + i and 32 + 16 h + i, i < 16; an eighth of them, which is exact, and the sign
+  // that follows commute with the rounding to FP32
+#pragma unroll
+  for (int i = 0; i < 16; ++i) {
+    const double sent = half ? e[i] : e[16 + i];
+    const double kept = half ? e[16 + i] : e[i];
+    const double got = __shfl_xor_sync(0xffffffffu, sent, 1);
+    const double a = half ? got : kept, b = half ? kept : got;
+    own[16 * half + i] = static_cast<float>((a + b) * 0.125);
+    own[32 + 16 * half + i] = static_cast<float>((a - b) * 0.125);
+  }
+}
+
+// kTurn: one output tile per CTA, with output transforms (TN = 2).
+template <int TN, bool kDump, bool kFused, bool kTurn>
 __global__ void __launch_bounds__(kThreads, 1)
 tmem_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constant__ CUtensorMap out_map, const GemmParams p) {
   using S = Layout<TN>;
@@ -560,7 +598,33 @@ tmem_gemm_kernel(const __grid_constant__ CUtensorMap x_map, const __grid_constan
         a_scale = token_scale();
       }
       // ---------------- epilogue -------------------------------------------------------
-      if (split_k > 1) {
+      if constexpr (kTurn) {
+        // The sums go to shared memory over the stage ring, whose last operands have been consumed.
+        constexpr int kRow = S::kCols + 1;
+        float* sums = reinterpret_cast<float*>(stages);
+#pragma unroll
+        for (int c = 0; c < kWarpCols / 2; ++c) unpack2(acc[c], sums[row * kRow + group * kWarpCols + 2 * c], sums[row * kRow + group * kWarpCols + 2 * c + 1]);
+        asm volatile("bar.sync 1, %0;" ::"n"(kDrainWarps * 32) : "memory");
+        const int turned = p.j_base + nb * TN + (warp & 1);  // tile row of this warp, of rows 16 (warp / 2) ..
+        const int64_t first = static_cast<int64_t>(mb) * kBM + (warp >> 1) * 16;
+        if (turned < p.n_j && first < p.m) {
+          float* region = sums + (warp >> 1) * 16 * kRow + (warp & 1) * kTile;
+          const int32_t* meta = p.u_metadata + static_cast<int64_t>(turned) * 4 * kTile;
+          turn_rows(region, kRow, meta, lane);
+          __syncwarp();
+          const bool identity = meta[0] == 0;
+          const int t_lo = identity ? lane : meta[kTile + lane], t_hi = identity ? lane + 32 : meta[kTile + lane + 32];
+          const int from_lo = (t_lo & 31) + (t_lo < 32 ? 0 : 32), from_hi = (t_hi & 31) + (t_hi < 32 ? 0 : 32);
+          const float left_lo = identity ? 1.0f : static_cast<float>(meta[2 * kTile + lane]);
+          const float left_hi = identity ? 1.0f : static_cast<float>(meta[2 * kTile + lane + 32]);
+          const int rows_here = p.m - first < 16 ? static_cast<int>(p.m - first) : 16;
+          for (int r = 0; r < rows_here; ++r) {
+            const int64_t o = (first + r) * p.row_stride + static_cast<int64_t>(turned) * kTile + lane;
+            store_any(p.out, p.out_dtype, o, region[r * kRow + from_lo] * left_lo);
+            store_any(p.out, p.out_dtype, o + 32, region[r * kRow + from_hi] * left_hi);
+          }
+        }
+      } else if (split_k > 1) {
         // split-K: the CTA's FP32 tile goes to shared memory (over the stage ring, whose last
         // operands have been consumed; rows padded by one float so that a warp writing one row
         // per lane hits 32 banks) for the exchange below
@@ -750,11 +814,15 @@ int set_shared_memory(int device) {
   static std::once_flag once[64];
   cudaError_t attr_status = cudaSuccess;
   std::call_once(once[device & 63], [&] {
-    const void* kernels[4] = {
-        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, false>),
-        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, true>),
-        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, true, false>),
-        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, true, true>)};
+    const void* kernels[8] = {
+        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, false, false>),
+        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, true, false>),
+        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, true, false, false>),
+        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, true, true, false>),
+        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, false, TN == 2>),
+        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, true, TN == 2>),
+        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, true, false, TN == 2>),
+        reinterpret_cast<const void*>(tmem_gemm_kernel<TN, true, true, TN == 2>)};
     for (const void* kernel : kernels) {
       if (attr_status == cudaSuccess) {
         attr_status = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Layout<TN>::kSmemBytes);
@@ -786,7 +854,7 @@ int resident_clusters(int split, int device) {
     config.attrs = attr;
     config.numAttrs = 1;
     if (set_shared_memory<TN>(device) != AQ_OK ||
-        cudaOccupancyMaxActiveClusters(&clusters, reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, true>), &config) != cudaSuccess) {
+        cudaOccupancyMaxActiveClusters(&clusters, reinterpret_cast<const void*>(tmem_gemm_kernel<TN, false, true, false>), &config) != cudaSuccess) {
       (void)cudaGetLastError();
       clusters = 0;
     }
@@ -817,14 +885,12 @@ int launch_shape(const CUtensorMap& x_map, const CUtensorMap& out_map, const Gem
   attr[1].val.programmaticStreamSerializationAllowed = 1;
   config.attrs = attr;
   config.numAttrs = use_dependent_launch() ? 2 : 1;
-  cudaError_t status;
-  if (dump) {
-    status = fused ? cudaLaunchKernelEx(&config, tmem_gemm_kernel<TN, true, true>, x_map, out_map, p)
-                   : cudaLaunchKernelEx(&config, tmem_gemm_kernel<TN, true, false>, x_map, out_map, p);
-  } else {
-    status = fused ? cudaLaunchKernelEx(&config, tmem_gemm_kernel<TN, false, true>, x_map, out_map, p)
-                   : cudaLaunchKernelEx(&config, tmem_gemm_kernel<TN, false, false>, x_map, out_map, p);
-  }
+  const bool turn = TN == 2 && split == 1 && p.u_metadata != nullptr;
+  const auto kernel = turn ? (dump ? (fused ? tmem_gemm_kernel<TN, true, true, TN == 2> : tmem_gemm_kernel<TN, true, false, TN == 2>)
+                                   : (fused ? tmem_gemm_kernel<TN, false, true, TN == 2> : tmem_gemm_kernel<TN, false, false, TN == 2>))
+                           : (dump ? (fused ? tmem_gemm_kernel<TN, true, true, false> : tmem_gemm_kernel<TN, true, false, false>)
+                                   : (fused ? tmem_gemm_kernel<TN, false, true, false> : tmem_gemm_kernel<TN, false, false, false>));
+  const cudaError_t status = cudaLaunchKernelEx(&config, kernel, x_map, out_map, p);
   return check_cuda(status, "tensor-memory GEMM launch");
 }
 
@@ -949,7 +1015,10 @@ int launch_tmem_gemm(const LinearArgs& a, const GemmPlan& plan, cudaStream_t str
   rc = encode_activation_map(&x_map, a.xq, a.m, a.n_k, kBM, 2);
   if (rc != AQ_OK) return rc;
   const int rows_at_once = plan.rows_per_pass;
-  const int tn = a.u_metadata != nullptr && plan.split == 1 ? 4 : plan.tn;  // a transformed row needs its 64 columns in one warp
+  // With transforms and one K range a row's 64 columns have to meet in one warp: in the stage ring where every CTA has
+  // only one 128-column tile, else (the ring belongs to the next tile) in the drain warps of a 256-column one.
+  int tn = plan.tn;
+  if (a.u_metadata != nullptr && plan.split == 1) tn = (a.m + kBM - 1) / kBM * ((plan.rows_per_pass + 1) / 2) <= sm_count ? 2 : 4;
   alignas(64) CUtensorMap out_map;
   rc = encode_result_map(&out_map, a.out, a.out_dtype, a.m, static_cast<int64_t>(a.n_j) * kTile, tn == 4 ? 64 : tn == 3 ? 16 : 32, 32);
   if (rc != AQ_OK) return rc;

@@ -71,7 +71,8 @@ AQ_API int aq_version(void);
  *                           (default), AQ_GEMM_TILE_PAIRED (128 columns, two K steps per hand-over),
  *                           AQ_GEMM_TILE_NARROW (192 columns), AQ_GEMM_TILE_WIDE (256 columns).
  *                           Results are bit-identical across the three.  (Layers with an output
- *                           transform and a single K range always run 256 columns wide.)
+ *                           transform and a single K range run 128 columns wide where that is at
+ *                           most one CTA per SM, else 256, whatever is set.)
  *   AQ_OPT_GEMM_SPLIT       number of K ranges of the GEMM (1..8), 0 = automatic (default); changes
  *                           the FP32 summation order as aq_linear_plan reports.
  *   AQ_OPT_DECODE_KERNEL    AQ_DECODE_KERNEL_AUTO (default); AQ_DECODE_KERNEL_CLUSTER: never use

@@ -10,6 +10,7 @@ import torch
 
 from alignquant_b200 import _lib
 from alignquant_b200.quantization.exact import metadata_stack
+from alignquant_b200.synthetic import synthetic_module_tensors
 from oracle import alignquant_oracle as oc
 from tests import helpers
 
@@ -270,3 +271,39 @@ def test_options_set_by_another_thread_meet_whole_calls(options):
         thread.join()
     ext.device_status()
     assert seen[0] > 0
+
+
+@pytest.mark.parametrize("tile", ["paired", "narrow", "wide", "auto"])
+@pytest.mark.parametrize("transforms", [False, True])
+@pytest.mark.parametrize("m,n,k", [(1190, 2368, 192), (700, 16448, 32768 // 4), (2100, 640, 320)])
+def test_gemm_many_tiles_per_cta_under_tile_scales(options, tile, transforms, m, n, k):
+    """Tile scales, transformed and plain tile rows mixed in one CTA, integer sums and every result type while a CTA walks
+    several output tiles (ragged last ones), against calls of 64 rows, which the kernel for few rows answers; the second
+    shape has more output tiles than SMs with every width."""
+    ext = options
+    n_j, n_k = n // 64, k // 64
+    t = synthetic_module_tensors(n, k, m)
+    weights = ext.prepare_weights(*(t[name] for name in ("state_bits", "w4_payload", "w4_scales", "w8_payload", "w8_scales",
+                                                         "w4_row_offsets", "w8_row_offsets")), n_k=n_k)
+    gen = torch.Generator(device="cuda").manual_seed(m + n)
+    x = torch.randn(m, k, generator=gen, device="cuda").to(torch.bfloat16)
+    xq, a_s = ext.alignquant_activation_quantize_cuda(x, None, scale_mode="tile")
+    u = metadata_stack([-1 if i % 3 == 1 else i + 1 for i in range(n_j)], "cuda") if transforms else None
+    ext.set_gemm_split(1)
+    few = dict(schedule="forced_prefill_m64", scale_mode="tile")
+    dumps = m * n_j * n_k < 1 << 21
+    for dtype in (torch.float32, torch.bfloat16, torch.float16):
+        ext.set_gemm_tile("auto")
+        want, sums = [], []
+        for row in range(0, m, 64):
+            rows = xq[row : row + 64]
+            part = torch.empty((rows.size(0), n_j, n_k, 64), dtype=torch.int32, device="cuda") if dumps else None
+            scales = a_s.reshape(-1, n_k)[row // 16 : (row + rows.size(0) + 15) // 16].contiguous()
+            want.append(ext.alignquant_linear_prepared(rows, scales, weights, u, output_dtype=dtype, acc_dump=part, **few))
+            sums.append(part)
+        ext.set_gemm_tile(tile)
+        dump = torch.empty((m, n_j, n_k, 64), dtype=torch.int32, device="cuda") if dumps else None
+        have = ext.alignquant_linear_prepared(xq, a_s, weights, u, output_dtype=dtype, acc_dump=dump, **few)
+        ext.device_status()
+        assert torch.equal(have, torch.cat(want))
+        assert not dumps or torch.equal(dump, torch.cat(sums))
