@@ -155,12 +155,15 @@ def test_gemm_all_cta_tiles(options, tile):
     assert np.array_equal(plain.cpu().numpy(), want)
 
 
+@pytest.mark.parametrize("tile", ["paired", "narrow", "wide", "auto"])
 @pytest.mark.parametrize("split", ["2", "3", "8"])
 @pytest.mark.parametrize("m", [40, 128, 200])
-def test_gemm_split_k_clusters(options, m, split):
-    """K ranges over a thread-block cluster: integer sums exact, FP32 in split order, output transform applied."""
+def test_gemm_split_k_clusters(options, m, split, tile):
+    """K ranges over a thread-block cluster, with every tile width and (automatic width, up to 128 rows) the kernel for few
+    rows: integer sums exact, FP32 in split order, output transform applied to those sums."""
     ext = options
     ext.set_gemm_split(int(split))
+    ext.set_gemm_tile(tile)
     n, k = 320, 2048
     weights, tiles, scales, xq, a_s, a_mk = _case(ext, m, n, k, "tile", seed=77 + m)
     n_j, n_k = n // 64, k // 64
@@ -171,15 +174,20 @@ def test_gemm_split_k_clusters(options, m, split):
     ext.device_status()
     xq_np = xq.cpu().numpy()
     assert np.array_equal(dump.cpu().numpy(), oc.tile_accumulators_c(xq_np, tiles))
-    assert np.array_equal(out.cpu().numpy(), oc.linear_fp32_c(xq_np, a_mk, tiles, scales, int(split), fused=True))
+    sums = oc.linear_fp32_c(xq_np, a_mk, tiles, scales, int(split), fused=True)
+    assert np.array_equal(out.cpu().numpy(), sums)
+    u = metadata_stack([-1 if i % 3 == 1 else i + 1 for i in range(n_j)], "cuda")
+    turned = ext.alignquant_linear_prepared(xq, a_s, weights, u, schedule="forced_prefill_m64")
+    ext.device_status()
+    exact = oc.inverse_output(sums, u.cpu().numpy())  # another order of the FP64 additions: the FP32 results are those or their neighbours
+    assert np.allclose(turned.cpu().numpy(), exact, rtol=2.0**-23, atol=2.0**-45 * np.abs(sums).max())
 
 
 @pytest.mark.parametrize("tile", ["paired", "narrow", "wide", "auto"])
 @pytest.mark.parametrize("m,n,k", [(1190, 2368, 192), (33, 2624, 32768), (1999, 1088, 64)])
 def test_gemm_many_tiles_per_cta_and_column_passes(options, tile, m, n, k):
     """More output tiles than SMs (a CTA walks several, with an odd number of K steps and ragged last
-    row and column blocks), a layer above the 64 MiB of expanded weights (several passes over its
-    columns) and a single K step; every result type through the tensor-map stores.  FP32 sums are
+    row and column blocks), the longest K and a single K step; every result type through the tensor-map stores.  FP32 sums are
     compared bit for bit, the 16-bit results with their rounding of them."""
     ext = options
     ext.set_gemm_tile(tile)
@@ -307,3 +315,23 @@ def test_gemm_many_tiles_per_cta_under_tile_scales(options, tile, transforms, m,
         ext.device_status()
         assert torch.equal(have, torch.cat(want))
         assert not dumps or torch.equal(dump, torch.cat(sums))
+
+
+def test_gemm_transforms_in_several_column_passes(options):
+    """A layer above the scratch: the second pass transforms with the metadata of its own tile rows."""
+    ext = options
+    n, k, m = 34816, 8192, 160
+    n_j, n_k = n // 64, k // 64
+    assert n_j * n_k * 4096 > 256 << 20
+    t = synthetic_module_tensors(n, k, 1)
+    weights = ext.prepare_weights(*(t[name] for name in ("state_bits", "w4_payload", "w4_scales", "w8_payload", "w8_scales",
+                                                         "w4_row_offsets", "w8_row_offsets")), n_k=n_k)
+    x = torch.randn(m, k, generator=torch.Generator(device="cuda").manual_seed(2), device="cuda").to(torch.bfloat16)
+    xq, a_s = ext.alignquant_activation_quantize_cuda(x, None, scale_mode="token")
+    ext.set_gemm_split(1)
+    for u in (None, metadata_stack([-1 if i % 3 == 1 else i + 1 for i in range(n_j)], "cuda")):
+        have = ext.alignquant_linear_prepared(xq, a_s, weights, u, scale_mode="token", output_dtype=torch.bfloat16)
+        want = [ext.alignquant_linear_prepared(xq[row : row + 64], a_s[row : row + 64], weights, u, scale_mode="token",
+                                               schedule="forced_prefill_m64", output_dtype=torch.bfloat16) for row in range(0, m, 64)]
+        assert torch.equal(have, torch.cat(want))
+    ext.device_status()
