@@ -8,11 +8,11 @@
 // multiply-add.  That drain, not the tensor pipe, bounds the kernel.
 //
 // What a drain costs (measured with resident operands, cycles per SM for the 128 x 256 results of
-// one K64 step): the arithmetic alone 375 (one I2F and half a packed FMA per result, i.e. 1.5
-// issue slots), with its tensor-memory loads 590 (a load occupies the register file's write port as
-// arithmetic does), with barriers and MMAs 680-750, the tensor pipe 248.  This kernel: 850 (1.27 POPS
-// at 16384 x 19456 x 2560; the version before it, which widened W4 tiles inside the GEMM and drained
-// with eight warps, 0.69).  What brought it there:
+// one K64 step, from event times at a nominal 1.92 GHz: good to some per cent): the arithmetic alone 375 (one I2F
+// and half a packed FMA per result, i.e. 1.5 issue slots, or 384 cycles), with its tensor-memory loads 590 (a load
+// occupies the register file's write port as arithmetic does), with barriers and MMAs 680-750, the tensor pipe
+// 248.  This kernel: 850 (16384 x 19456 x 2560 with quantizer and expansion 1.15 POPS; the version before it, which
+// widened W4 tiles inside the GEMM and drained with eight warps, 0.67).  What brought it there:
 //   * sixteen drain warps, four per scheduler, each owning 32 rows x 16 TN columns: a warp that
 //     waits for a barrier or a tensor-memory load leaves its scheduler to three others (eight
 //     warps with twice the columns: 1040-1090 cycles per step);
@@ -22,7 +22,8 @@
 //     lane and a shuffle costs 2.5 times as much (436 against 178 cycles per step for the bare
 //     hand-over), a branch around the arrival 80 cycles per step;
 //   * the loop's registers: sums, loaded columns and little else (scales come from a ring in shared
-//     memory), so that nothing is spilled;
+//     memory).  The 128- and 192-column kernels spill nothing, the 256-column one some 90 bytes; an instantiation of it
+//     without the output transform spills 68 and is slower (16384 x 19456 x 2560 1381 -> 1446 us);
 //   * no work for single warps: next to sixteen busy warps an ordinary instruction of a single warp
 //     takes 5 to 10 cycles, so a warp that issues copies or widens tiles step by step falls behind
 //     the drain.  Hence two copies per stage and the expansion in a pass of its own.

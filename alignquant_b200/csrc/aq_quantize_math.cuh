@@ -33,9 +33,9 @@ __device__ __forceinline__ uint32_t pack4(int a, int b, int c, int d) {
 // callers' inv is 1 / scale to 2^-24 of it (one rounding) and |v / scale| <= 128, so v * inv is off by 2^-17, the
 // distance by 2^-26 more and, where `exact` rounds the quotient to FP32 first, that by 2^-18: below 0.5 - 2^-16 the
 // code is that of `exact` and lies in its range.  Otherwise (and for NaN) all four go to `exact`.  Every value
-// that goes there counts in a launch of two microseconds (with 1e-4 in place of 2^-16: 32 x 5120 bf16 2.5, now 1.9).  Full-rate instructions only:
-// conversions to and from integers run at a quarter of the rate and, with the compares, clamps and
-// masks of quantize_token_value, bounded the quantizers (8192 x 8192 bf16: 59 us).
+// that goes there counts in a launch of two microseconds (with 1e-4 in place of 2^-16: 32 x 5120 bf16 2.5, now 1.9).
+// Full-rate instructions only: conversions of floats to integers run at a fraction of the rate and, with the
+// compares, clamps and masks of quantize_token_value, bounded the quantizers (8192 x 8192 bf16: 59 us).
 template <typename Exact>
 __device__ __forceinline__ uint32_t quantize4(float v0, float v1, float v2, float v3, float inv, Exact exact) {
   constexpr float kMagic = 12582912.0f, kClear = 0.5f - 1.0f / 65536.0f;
